@@ -388,7 +388,7 @@ class GpuCSCMapping:
 
     ``value_layout``: the element values the assembly writes and gathers --
     ``"block"`` (default: per tet the 2x2 blocks of its 55 entity pairs, one
-    4-byte record and one contiguous read per four entries of A) or
+    8-byte record per four entries of A and one contiguous read per tet) or
     ``"packed"`` (the canonical upper triangle, one record per two entries,
     ``record_bytes`` 8 or 4). A is bit for bit the same in both."""
 

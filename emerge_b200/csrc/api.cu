@@ -290,6 +290,7 @@ int emg_assemble_batch(const emg_assembly_job *h_jobs, int n_jobs, int precision
   const int kind = h_jobs[0].mat.kind;
   const int layout = h_jobs[0].plan ? h_jobs[0].plan->value_layout : EMG_LAYOUT_PACKED;
   ecta[0] = gcta[0] = 0;
+  bool wide = true;
   for (int i = 0; i < n_jobs; ++i) {
     const emg_assembly_job &j = h_jobs[i];
     const emg_plan *p = j.plan;
@@ -303,9 +304,10 @@ int emg_assemble_batch(const emg_assembly_job *h_jobs, int n_jobs, int precision
     ea[i] = ElemArgs{j.d_nodes, j.n_nodes, j.d_tets, p->n_tets, j.d_tetids, p->n_assy, j.mat.d_er, j.mat.d_ur,
                      j.alpha_re, j.alpha_im, j.beta_re, j.beta_im, j.d_values, j.d_status};
     ecta[i + 1] = ecta[i] + (p->n_assy + 127) / 128;
-    int rc = gather_job_fill(p, j.d_plan, j.d_indptr, j.d_values, j.d_A, &ga[i]);
+    int rc = gather_job_fill(p, j.d_plan, j.d_indptr, j.d_values, j.d_A, precision, &ga[i]);
     if (rc) return rc;
     gcta[i + 1] = gcta[i] + (p->n_ent > 0 ? ga[i].n_ctas : 0);
+    wide = wide && ga[i].wide;
   }
   CUDA_TRY(cudaMemcpyAsync(d_table, h_table, batch_offset(n_jobs, 4), cudaMemcpyHostToDevice, S(stream)));
   const char *d = static_cast<const char *>(d_table);
@@ -315,7 +317,7 @@ int emg_assemble_batch(const emg_assembly_job *h_jobs, int n_jobs, int precision
   if (rc) return rc;
   return launch_gather_batch(reinterpret_cast<const GatherJob *>(d + batch_offset(n_jobs, 2)),
                              reinterpret_cast<const int64_t *>(d + batch_offset(n_jobs, 3)), n_jobs, gcta[n_jobs],
-                             precision, layout, S(stream));
+                             wide, precision, layout, S(stream));
 }
 
 int emg_form_sweep(const void *d_K, const void *d_M, const void *d_P, int64_t nnz, const double *h_coef, int nf,

@@ -73,6 +73,18 @@ __host__ __device__ __forceinline__ constexpr int ent_dof2(int i) { return i < 6
 // Block gather record: ia * 55 + block_index(min(a, b), max(a, b)) of row
 // entity a and column entity b, bit 31 set when a > b (the block is stored
 // transposed: its middle two values swap).
+// A row pair's record is two of them (uint2), in item order, both stored the
+// same way round; kBlockNone where there are fewer. A longer list, or one of two
+// blocks stored different ways round, has y = kBlockLong and x = its word offset
+// in the chunk's records | length << 16, or x = 0 when it is an entity's pair
+// with itself. A chunk of I items has kPairWords * I words from word
+// kPairWords * (its first item): its H row pairs' records, then per item the
+// entity's block with itself, then the other long lists. That is enough: an
+// entity of I items with h1, h2, h3 row pairs of one block, of two and with a
+// long list beside its own, r3 >= 2 h3 blocks in the long lists, has
+// 9 I = h1 + 2 h2 + r3 and needs 2 (1 + h1 + h2 + h3) + I + r3 <= 2 + 19 I words.
+constexpr int kPairWords = 22;
+constexpr uint32_t kBlockNone = 0xffffffffu, kBlockLong = 0xfffffffeu;  // block numbers end below both
 __host__ __device__ __forceinline__ bool block_record_fits(int64_t n_assy) { return n_assy * 55 < (1LL << 31); }
 
 // Compact gather record (emg_plan.record_bytes = 4; one uint32 per
@@ -141,13 +153,14 @@ struct ElemArgs {
 // one job of a batched packed gather (emg_gather_batch)
 struct GatherJob {
   const int32_t *ent_ptr, *order;
-  const void *pidx;       // packed: int2 records; block: uint32 block records
-  const uint16_t *posoff; // packed: list start per position; block: per row pair
+  const void *pidx;       // packed: int2 records; block: row-pair records
+  const uint16_t *posoff; // packed: list start per position
   const int32_t *indptr;
-  const uint32_t *ent_cnt;  // block layout: adjacent edges | faces << 16 per entity
+  const struct ChunkDesc *desc;  // block layout
   const void *values;
   double2 *A;
   int64_t E, F, n_values, n_ctas;  // n_values: value slots (packed) or blocks (block layout)
+  int64_t wide;                    // block layout: the values are aligned to half a block
 };
 
 // Gather chunks: a warp owns CHUNK consecutive entities of one kind. Their
@@ -156,6 +169,19 @@ struct GatherJob {
 constexpr int CHUNK = 8;
 constexpr int CHUNK_MAX_POS = 1024;   // positions per run of a chunk (plan capacity)
 constexpr int CHUNK_MAX_ITEMS = 1023; // items per chunk (10-bit item index)
+
+// A chunk as the block gather reads it: one 64-byte record per chunk, in
+// processing order, so that a CTA knows its chunk after one load.
+struct __align__(64) ChunkDesc {
+  int32_t I0, A0, A1;      // first item; starts of its two runs of A
+  uint16_t H, nI;          // row pairs, items
+  uint16_t hs[CHUNK];      // first row pair of each entity (H for entities past the chunk's last)
+  uint8_t ne[CHUNK];       // adjacent edges of each entity
+  uint8_t cnt[CHUNK];      // items of each entity
+  uint8_t self[CHUNK];     // the entity's rank among its adjacent edges (faces)
+  uint8_t faces, pad[7];   // 1: a chunk of faces
+};
+static_assert(sizeof(ChunkDesc) == 64, "chunk descriptor must be 64 bytes");
 
 __host__ __device__ __forceinline__ int64_t n_edge_chunks(int64_t E) { return (E + CHUNK - 1) / CHUNK; }
 __host__ __device__ __forceinline__ int64_t n_chunks(int64_t E, int64_t F) {
@@ -236,9 +262,9 @@ int launch_gather(const emg_plan *p, const void *d_plan, const int32_t *indptr, 
                   int precision, int layout, double ar, double ai, double br, double bi, void *A, int64_t *st,
                   cudaStream_t s);
 int gather_job_fill(const emg_plan *p, const void *d_plan, const int32_t *d_indptr, const void *d_values, void *d_A,
-                    GatherJob *out);
+                    int precision, GatherJob *out);
 int launch_gather_batch(const GatherJob *d_jobs, const int64_t *d_cta_start, int n_jobs, int64_t total_ctas,
-                        int precision, int layout, cudaStream_t s);
+                        bool wide, int precision, int layout, cudaStream_t s);
 int launch_form_sweep(const void *K, const void *M, const void *P, int64_t nnz, const double *coef, int nf,
                       void *out, int64_t stride, cudaStream_t s);
 int launch_form_batch(const emg_form_item *items, const int64_t *tile_start, const int32_t *n_items, int max_items,

@@ -251,100 +251,188 @@ __global__ void __launch_bounds__(PackedShape<R, COMPACT>::warps * 32, PackedSha
   gather_packed_chunk<R, COMPACT>(m, pidx_v, posoff, n_values, v, ar, ai, A, slot2);
 }
 
-// ---- entity-pair block layout (EMG_LAYOUT_BLOCK). A lane owns a row pair of
-// the chunk's first-DoF runs -- the first-DoF row p of an adjacent entity and
-// its partner row p' (the entity's second DoF) -- and sums, over the tets of
-// its list in item order, the 2x2 blocks of that entity pair: the entries of
-// rows p, p' in the chunk entity's two columns. One 4-byte record and one
-// contiguous 64-byte (32-byte) read give four entries of A; every entry sums
-// the same values in the same order as the packed gather.
-constexpr int BG_WARPS = 4;
+// ---- entity-pair block layout (EMG_LAYOUT_BLOCK). A row pair of a chunk's
+// first-DoF run -- the first-DoF row p of an adjacent entity and its partner
+// row p' (the entity's second DoF) -- gets four entries of A, the sums over its
+// tets, in item order, of the 2x2 blocks of that entity pair.
+//
+// A CTA gathers one chunk. Two lanes share a row pair, half a block (two values,
+// one 32-byte or, complex64, 16-byte load) each. Two different entities of a
+// conforming mesh share at most two tets, so a row pair's record is two block
+// numbers, loaded without a list start, and every lane has four loads in
+// flight; only an entity's pair with itself (5-6 tets around an edge) is
+// longer, and its list has a known place. Chain of dependent loads per chunk:
+// descriptor, records, values.
+//
+// A lane per row pair that walked its list ran as long as the warp's longest
+// list, 5-6 dependent record -> value loads where the mean list has 1.4: 1,008,000
+// tets took 2,380 us complex128 and 1,850 complex64; now 1,600 and 1,402. Bound:
+// HBM for complex128 (10.2 GB, 6.4 TB/s), latency for complex64 (5.0 TB/s).
+// Two warps per CTA and 18 CTAs per SM (56 registers): 16 CTAs 1,653 / 1,447,
+// 20 (spills) 1,793 / 1,445; one warp 1,812 / 1,488, four 1,761 / 1,544. Four
+// lanes per row pair: 2,069 / 1,790. The chunk's runs of A staged in shared
+// memory and written by bulk copies: 1,849 / 1,608 -- the stage takes the L1 that
+// holds the loads in flight -- and with the chunks pipelined through cp.async, up
+// to eight per CTA: 2,082 / 1,738.
+constexpr int BG_WARPS = 2;
+constexpr int BG_CTAS = 18;  // per SM
 
+// value q (0..3) of the stored block of record r, or zero
 template <typename R>
-__device__ __forceinline__ void gather_block_chunk(const ChunkMeta &m, const uint32_t *brec, const uint16_t *hoff,
-                                                   const int32_t *indptr, const uint32_t *ent_cnt, int64_t n_blocks,
-                                                   const void *v, double ar, double ai, double2 *A,
-                                                   int32_t *se /* 3 * CHUNK + 1 ints of this warp */) {
-  const int lane = threadIdx.x & 31;
-  int32_t *hs = se;                  // half start of entity e in the chunk, hs[nx] = all row pairs
-  int32_t *nes = se + CHUNK + 1;     // adjacent edges of entity e
-  int32_t *cs = se + 2 * CHUNK + 1;  // first-DoF column start of entity e, relative to A0
-  if (lane < m.nx) {
-    const int32_t c = indptr[m.cb0 + lane] - m.A0;
-    cs[lane] = c;
-    hs[lane] = c / 2;
-    nes[lane] = (int32_t)(ent_cnt[m.x0 + lane] & 0xffffu);
-  }
-  if (lane == 0) hs[m.nx] = m.Lsum / 2;
-  __syncwarp();
-  const uint64_t pv = policy_evict_last();
-  const int H = m.Lsum / 2;
-  const int total = 10 * (m.I1 - m.I0);
-  const uint32_t *rl = brec + (int64_t)10 * m.I0;
-  const int64_t hb = m.hbase / 2;
-  int e = 0;
-  // list bounds of the lane's next row pair are loaded while the current one is summed
-  // complex64 values: the first record of the lane's next row pair is also
-  // loaded ahead (measured 2% faster; slower for complex128)
-  constexpr bool RECORD_AHEAD = !std::is_same<R, double>::value;
-  int n0 = 0, n1 = 0;
-  uint32_t r0n = 0;
-  if (lane < H) {
-    n0 = hoff[hb + lane];
-    n1 = lane + 1 < H ? (int)hoff[hb + lane + 1] : total;
-    if (RECORD_AHEAD && n0 < min(n1, total)) r0n = __ldg(rl + n0);
-  }
-  for (int h = lane; h < H; h += 32) {
-    while (e + 1 < m.nx && h >= hs[e + 1]) ++e;  // h only grows along a lane
-    const int hl = h - hs[e], ne = nes[e];
-    const int nf = hs[e + 1] - hs[e] - ne;
-    const int p = hl < ne ? cs[e] + hl : cs[e] + ne + hl;
-    const int pp = hl < ne ? p + ne : p + nf;
-    const int o0 = n0;
-    const int o1 = min(n1, total);
-    const uint32_t r0 = r0n;
-    if (h + 32 < H) {
-      n0 = hoff[hb + h + 32];
-      n1 = h + 33 < H ? (int)hoff[hb + h + 33] : total;
-    }
-    double s0r = 0.0, s0i = 0.0, s1r = 0.0, s1i = 0.0, s2r = 0.0, s2i = 0.0, s3r = 0.0, s3i = 0.0;
-    for (int k = o0; k < o1; ++k) {
-      const uint32_t rec = (RECORD_AHEAD && k == o0) ? r0 : __ldg(rl + k);
-      const int64_t b = rec & 0x7fffffffu;
-      if (b >= n_blocks) continue;  // only a plan whose build was flagged can hold this
-      const C64 u0 = load_val_last<R>(v, 4 * b, pv), u3 = load_val_last<R>(v, 4 * b + 3, pv);
-      C64 u1 = load_val_last<R>(v, 4 * b + 1, pv), u2 = load_val_last<R>(v, 4 * b + 2, pv);
-      if (rec >> 31) {
-        const C64 t = u1;
-        u1 = u2;
-        u2 = t;
-      }
-      s0r += u0.re;
-      s0i += u0.im;
-      s1r += u1.re;
-      s1i += u1.im;
-      s2r += u2.re;
-      s2i += u2.im;
-      s3r += u3.re;
-      s3i += u3.im;
-    }
-    if (RECORD_AHEAD && h + 32 < H && n0 < min(n1, total)) r0n = __ldg(rl + n0);
-    A[m.A0 + p] = make_double2(ar * s0r - ai * s0i, ar * s0i + ai * s0r);
-    A[m.A1 + p] = make_double2(ar * s1r - ai * s1i, ar * s1i + ai * s1r);
-    A[m.A0 + pp] = make_double2(ar * s2r - ai * s2i, ar * s2i + ai * s2r);
-    A[m.A1 + pp] = make_double2(ar * s3r - ai * s3i, ar * s3i + ai * s3r);
+__device__ __forceinline__ C64 load_block_value(const void *v, uint32_t r, int q, uint32_t n_blocks, uint64_t pol) {
+  const uint32_t b = r & 0x7fffffffu;
+  if (b >= n_blocks) return {0.0, 0.0};  // no block (kBlockNone), or a plan whose build was flagged
+  // bit 31: stored transposed, the middle two values swap
+  return load_val_last<R>(v, 4 * (int64_t)b + (((r >> 31) && (q == 1 || q == 2)) ? 3 - q : q), pol);
+}
+
+// half y of block b: its values 2y and 2y + 1 (v_y: the values' start plus y
+// halves); WIDE: one load, which needs the values aligned to half a block
+template <typename R, bool WIDE>
+__device__ __forceinline__ void load_half_block(const char *v_y, uint32_t b, uint32_t n_blocks, uint64_t pol, R u[4]) {
+  u[0] = u[1] = u[2] = u[3] = 0;
+  if (b >= n_blocks) return;
+  const char *p = v_y + (uint64_t)b * (8 * sizeof(R));
+  if constexpr (!WIDE) {
+    const C64 a = load_val_last<R>(p, 0, pol), c = load_val_last<R>(p, 1, pol);
+    u[0] = (R)a.re, u[1] = (R)a.im, u[2] = (R)c.re, u[3] = (R)c.im;
+  } else if constexpr (sizeof(R) == 8) {
+    asm volatile("ld.global.nc.L2::cache_hint.v4.f64 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=d"(u[0]), "=d"(u[1]), "=d"(u[2]), "=d"(u[3])
+                 : "l"(p), "l"(pol));
+  } else {
+    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(u[0]), "=f"(u[1]), "=f"(u[2]), "=f"(u[3])
+                 : "l"(p), "l"(pol));
   }
 }
 
+// The chunk's entities' pairs with themselves (lists of more than two), one
+// warp: a quad of lanes per entity, one value of the block each, eight blocks
+// in flight, added in list order.
 template <typename R>
-__global__ void __launch_bounds__(BG_WARPS * 32, 10)
-    k_gather_block(const int32_t *ent_ptr, const int32_t *order, const uint32_t *brec, const uint16_t *hoff,
-                   const uint32_t *ent_cnt, int64_t E, int64_t F, int64_t n_blocks, const int32_t *indptr,
-                   const void *v, double ar, double ai, double2 *A) {
-  __shared__ int32_t se[BG_WARPS][3 * CHUNK + 1];
-  ChunkMeta m;
-  if (!chunk_meta(ent_ptr, order, indptr, E, F, (int64_t)blockIdx.x * BG_WARPS + (threadIdx.x >> 5), m)) return;
-  gather_block_chunk<R>(m, brec, hoff, indptr, ent_cnt, n_blocks, v, ar, ai, A, se[threadIdx.x >> 5]);
+__device__ __forceinline__ void gather_self_pairs(const ChunkDesc &d, const uint32_t *self, uint32_t n_blocks,
+                                                  const void *v, double ar, double ai, uint64_t pol, double2 *A) {
+  const int lane = threadIdx.x & 31, q = lane & 3, e = lane >> 2, H = d.H;
+  const int n = d.cnt[e];
+  for (int k = 0; k < e; ++k) self += d.cnt[k];
+  double sr = 0.0, si = 0.0;
+  for (int k0 = 0; __any_sync(0xffffffffu, n > 2 && k0 < n); k0 += 8) {
+    const uint32_t r0 = k0 + q < n ? __ldg(self + k0 + q) : kBlockNone;
+    const uint32_t r1 = k0 + q + 4 < n ? __ldg(self + k0 + q + 4) : kBlockNone;
+    R u[8][2];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t r = __shfl_sync(0xffffffffu, k < 4 ? r0 : r1, (lane & 28) | (k & 3));
+      const C64 t = load_block_value<R>(v, r, q, n_blocks, pol);
+      u[k][0] = (R)t.re, u[k][1] = (R)t.im;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      sr += (double)u[k][0];
+      si += (double)u[k][1];
+    }
+  }
+  if (n > 2) {
+    const int ne = d.ne[e], nf = (e + 1 < CHUNK ? d.hs[e + 1] : H) - d.hs[e] - ne;
+    const int p = 2 * d.hs[e] + (d.faces ? 2 * ne : 0) + d.self[e] + ((q & 2) ? (d.faces ? nf : ne) : 0);
+    if (p < 2 * H) A[((q & 1) ? d.A1 : d.A0) + p] = make_double2(ar * sr - ai * si, ar * si + ai * sr);
+  }
+}
+
+template <typename R, bool WIDE>
+__device__ __forceinline__ void gather_block_chunk(const ChunkDesc *desc, const uint32_t *brec, uint32_t n_blocks,
+                                                   const void *v, double ar, double ai, double2 *A) {
+  __shared__ ChunkDesc d;
+  if (threadIdx.x < sizeof(ChunkDesc) / 4)
+    reinterpret_cast<uint32_t *>(&d)[threadIdx.x] = __ldg(reinterpret_cast<const uint32_t *>(desc) + threadIdx.x);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, y = lane & 1;
+  const int H = d.H, to_A1 = d.A1 - d.A0;
+  double2 *A0 = A + d.A0;
+  const uint64_t pol = policy_evict_last();
+  const char *v_y = static_cast<const char *>(v) + y * 4 * sizeof(R);
+  const uint32_t *words = brec + (int64_t)kPairWords * d.I0;
+  const uint2 *pairs = reinterpret_cast<const uint2 *>(words);
+  const uint2 none = make_uint2(kBlockNone, kBlockNone);
+  uint2 nxt = threadIdx.x < H ? __ldg(pairs + threadIdx.x) : none;
+  if (w == BG_WARPS - 1) gather_self_pairs<R>(d, words + 2 * H, n_blocks, v, ar, ai, pol, A);
+
+  for (int h0 = 32 * w; h0 < H; h0 += 32 * BG_WARPS) {
+    const int h = h0 + lane;
+    uint2 pr = nxt;  // the next records are loaded while these are summed
+    nxt = h + 32 * BG_WARPS < H ? __ldg(pairs + h + 32 * BG_WARPS) : none;
+    // the row pair's first row p in the run, p' - p, transposed
+    uint32_t pk = 0;
+    if (h < H) {
+      int x = h >= d.hs[4] ? 4 : 0;
+      x += h >= d.hs[x + 2] ? 2 : 0;
+      x += h >= d.hs[x + 1] ? 1 : 0;
+      const int hb = d.hs[x], hl = h - hb, ne = d.ne[x], nf = (x + 1 < CHUNK ? d.hs[x + 1] : H) - hb - ne;
+      pk = (uint32_t)(hl < ne ? h + hb : h + hb + ne) | ((uint32_t)(hl < ne ? ne : nf) << 16) | (pr.x & 0x80000000u);
+    }
+    const bool is_long = pr.y == kBlockLong;
+    // longer lists of two different entities: only a mesh that is not
+    // conforming has any, so they are summed one by one
+    unsigned longs = __ballot_sync(0xffffffffu, is_long && pr.x != 0);
+    while (longs) {
+      const int src = __ffs(longs) - 1;
+      longs &= longs - 1;
+      const uint32_t x = __shfl_sync(0xffffffffu, pr.x, src), z = __shfl_sync(0xffffffffu, pk, src);
+      if (lane < 4) {
+        const int off = (int)(x & 0xffffu), end = min(off + (int)(x >> 16), kPairWords * (int)d.nI);
+        double sr = 0.0, si = 0.0;
+        for (int i = off; i < end; ++i) {
+          const C64 u = load_block_value<R>(v, __ldg(words + i), lane, n_blocks, pol);
+          sr += u.re;
+          si += u.im;
+        }
+        const int p = (int)(z & 0xffffu) + ((lane & 2) ? (int)((z >> 16) & 0x7fffu) : 0);
+        A0[((lane & 1) ? to_A1 : 0) + p] = make_double2(ar * sr - ai * si, ar * si + ai * sr);
+      }
+    }
+    if (h >= H || is_long) pk = 0xffffu;  // nothing to store
+    if (is_long) pr = none;
+    R u[2][2][4];
+    uint32_t at[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int src = 16 * j + (lane >> 1);
+      load_half_block<R, WIDE>(v_y, __shfl_sync(0xffffffffu, pr.x, src) & 0x7fffffffu, n_blocks, pol, u[j][0]);
+      load_half_block<R, WIDE>(v_y, __shfl_sync(0xffffffffu, pr.y, src) & 0x7fffffffu, n_blocks, pol, u[j][1]);
+      at[j] = __shfl_sync(0xffffffffu, pk, src);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int p = at[j] & 0xffffu, dp = (at[j] >> 16) & 0x7fffu;
+      const bool tr = at[j] >> 31;
+      // values 2y, 2y + 1 belong to row y and columns 0, 1, or, transposed, to column y and rows 0, 1
+      double2 *o = A0 + p + (y ? (tr ? to_A1 : dp) : 0);
+      const int step = tr ? dp : to_A1;
+      if (p != 0xffffu)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          double sr = 0.0, si = 0.0;
+          sr += (double)u[j][0][2 * k];
+          si += (double)u[j][0][2 * k + 1];
+          sr += (double)u[j][1][2 * k];
+          si += (double)u[j][1][2 * k + 1];
+          o[k * step] = make_double2(ar * sr - ai * si, ar * si + ai * sr);
+        }
+    }
+  }
+}
+
+template <typename R, bool WIDE>
+__global__ void __launch_bounds__(BG_WARPS * 32, BG_CTAS)
+    k_gather_block(const ChunkDesc *desc, const uint32_t *brec, uint32_t n_blocks, const void *v, double ar, double ai,
+                   double2 *A) {
+  gather_block_chunk<R, WIDE>(desc + blockIdx.x, brec, n_blocks, v, ar, ai, A);
+}
+
+// whether the values can be read half a block at a time
+static bool half_block_aligned(const void *v, bool f32) {
+  return reinterpret_cast<uintptr_t>(v) % (f32 ? 16 : 32) == 0;
 }
 
 // Several jobs' packed gathers (8-byte records, alpha = 1) in one launch: job
@@ -370,10 +458,9 @@ __global__ void __launch_bounds__(PackedShape<R, false>::warps * 32, PackedShape
 }
 
 // Several jobs' block gathers (alpha = 1) in one launch, as k_gather_packed_batch.
-template <typename R>
-__global__ void __launch_bounds__(BG_WARPS * 32, 10)
+template <typename R, bool WIDE>
+__global__ void __launch_bounds__(BG_WARPS * 32, BG_CTAS)
     k_gather_block_batch(const GatherJob *jobs, const int64_t *cta_start, int n_jobs) {
-  __shared__ int32_t se[BG_WARPS][3 * CHUNK + 1];
   const int64_t b = blockIdx.x;
   int lo = 0, hi = n_jobs - 1;
   while (lo < hi) {
@@ -383,11 +470,8 @@ __global__ void __launch_bounds__(BG_WARPS * 32, 10)
   }
   if (n_jobs <= 0 || b >= cta_start[n_jobs]) return;
   const GatherJob &j = jobs[lo];
-  ChunkMeta m;
-  if (!chunk_meta(j.ent_ptr, j.order, j.indptr, j.E, j.F, (b - cta_start[lo]) * BG_WARPS + (threadIdx.x >> 5), m))
-    return;
-  gather_block_chunk<R>(m, static_cast<const uint32_t *>(j.pidx), j.posoff, j.indptr, j.ent_cnt, j.n_values,
-                        j.values, 1.0, 0.0, j.A, se[threadIdx.x >> 5]);
+  gather_block_chunk<R, WIDE>(j.desc + (b - cta_start[lo]), static_cast<const uint32_t *>(j.pidx),
+                              (uint32_t)j.n_values, j.values, 1.0, 0.0, j.A);
 }
 
 // ---------------------------------------------------------------------------
@@ -498,16 +582,17 @@ int launch_gather(const emg_plan *p, const void *d_plan, const int32_t *d_indptr
   if (layout == EMG_LAYOUT_BLOCK) {
     if (two) return fail(EMG_EINVAL, "the block layout takes one value array");
     const uint32_t *brec = reinterpret_cast<const uint32_t *>(plan + p->off_pidx);
-    const uint16_t *hoff = reinterpret_cast<const uint16_t *>(plan + p->off_hoff);
-    const uint32_t *ent_cnt = reinterpret_cast<const uint32_t *>(plan + p->off_ent_cnt);
-    const int gb = grid_for(n_chunks(p->n_edges, p->n_tris), BG_WARPS);
-    const int64_t nb = p->n_assy * 55;
-    if (f32)
-      k_gather_block<float><<<gb, BG_WARPS * 32, 0, s>>>(ent_ptr, order, brec, hoff, ent_cnt, p->n_edges, p->n_tris,
-                                                          nb, d_indptr, d_v1, ar, ai, A);
-    else
-      k_gather_block<double><<<gb, BG_WARPS * 32, 0, s>>>(ent_ptr, order, brec, hoff, ent_cnt, p->n_edges,
-                                                           p->n_tris, nb, d_indptr, d_v1, ar, ai, A);
+    const ChunkDesc *desc = reinterpret_cast<const ChunkDesc *>(plan + p->off_hoff);
+    const unsigned nch = (unsigned)n_chunks(p->n_edges, p->n_tris);
+    const uint32_t nb = (uint32_t)(p->n_assy * 55);  // below 2^31: block_record_fits
+#define EMG_BG(R, W) k_gather_block<R, W><<<nch, BG_WARPS * 32, 0, s>>>(desc, brec, nb, d_v1, ar, ai, A)
+    const bool wide = half_block_aligned(d_v1, f32);
+    if (f32) {
+      if (wide) EMG_BG(float, true); else EMG_BG(float, false);
+    } else {
+      if (wide) EMG_BG(double, true); else EMG_BG(double, false);
+    }
+#undef EMG_BG
     return launch_check("k_gather_block");
   }
   if (layout == EMG_LAYOUT_PACKED) {
@@ -540,7 +625,7 @@ int launch_gather(const emg_plan *p, const void *d_plan, const int32_t *d_indptr
 }
 
 int gather_job_fill(const emg_plan *p, const void *d_plan, const int32_t *d_indptr, const void *d_values, void *d_A,
-                    GatherJob *out) {
+                    int precision, GatherJob *out) {
   const bool block = p->value_layout == EMG_LAYOUT_BLOCK;
   if (!block && p->record_bytes != 8)
     return fail(EMG_EINVAL, "batched gathers take block-layout plans or packed ones with 8-byte records");
@@ -548,28 +633,33 @@ int gather_job_fill(const emg_plan *p, const void *d_plan, const int32_t *d_indp
   out->ent_ptr = reinterpret_cast<const int32_t *>(plan + p->off_ent_ptr);
   out->order = reinterpret_cast<const int32_t *>(plan + p->off_order);
   out->pidx = plan + p->off_pidx;
-  out->posoff = reinterpret_cast<const uint16_t *>(plan + (block ? p->off_hoff : p->off_posoff));
+  out->posoff = reinterpret_cast<const uint16_t *>(plan + p->off_posoff);
   out->indptr = d_indptr;
-  out->ent_cnt = reinterpret_cast<const uint32_t *>(plan + p->off_ent_cnt);
+  out->desc = reinterpret_cast<const ChunkDesc *>(plan + p->off_hoff);
   out->values = d_values;
   out->A = static_cast<double2 *>(d_A);
   out->E = p->n_edges;
   out->F = p->n_tris;
   out->n_values = p->n_assy * (block ? 55 : 210);
-  const int warps = block ? BG_WARPS : PackedShape<double, false>::warps;
-  out->n_ctas = (n_chunks(p->n_edges, p->n_tris) + warps - 1) / warps;
+  const int per_cta = block ? 1 : PackedShape<double, false>::warps;  // chunks
+  out->n_ctas = (n_chunks(p->n_edges, p->n_tris) + per_cta - 1) / per_cta;
+  out->wide = block && half_block_aligned(d_values, values_fp32(precision));
   return EMG_OK;
 }
 
 int launch_gather_batch(const GatherJob *d_jobs, const int64_t *d_cta_start, int n_jobs, int64_t total_ctas,
-                        int precision, int layout, cudaStream_t s) {
+                        bool wide, int precision, int layout, cudaStream_t s) {
   if (n_jobs == 0 || total_ctas == 0) return EMG_OK;
   if (total_ctas > INT32_MAX) return fail(EMG_ERANGE, "too many CTAs (%lld)", (long long)total_ctas);
   if (layout == EMG_LAYOUT_BLOCK) {
-    if (values_fp32(precision))
-      k_gather_block_batch<float><<<(unsigned)total_ctas, BG_WARPS * 32, 0, s>>>(d_jobs, d_cta_start, n_jobs);
-    else
-      k_gather_block_batch<double><<<(unsigned)total_ctas, BG_WARPS * 32, 0, s>>>(d_jobs, d_cta_start, n_jobs);
+#define EMG_BGB(R, W) \
+  k_gather_block_batch<R, W><<<(unsigned)total_ctas, BG_WARPS * 32, 0, s>>>(d_jobs, d_cta_start, n_jobs)
+    if (values_fp32(precision)) {
+      if (wide) EMG_BGB(float, true); else EMG_BGB(float, false);
+    } else {
+      if (wide) EMG_BGB(double, true); else EMG_BGB(double, false);
+    }
+#undef EMG_BGB
     return launch_check("k_gather_block_batch");
   }
   static_assert(PackedShape<double, false>::warps == PackedShape<float, false>::warps, "same chunks per CTA");

@@ -398,84 +398,138 @@ __global__ void __launch_bounds__(CC_WARPS * 32)
   }
 }
 
-// Block gather lists (EMG_LAYOUT_BLOCK), warp per chunk: every (item, row
-// entity) of the chunk contributes the tet's block of that entity pair to one
-// row pair (the row entity's first-DoF row and its partner row, which hold the
-// same tets); counted per row pair, scanned into hoff (list start relative to
-// the chunk's first record, 10 * I0), then placed in item order, so each
-// output sums its contributions in the order of the packed lists.
+// Block gather records (EMG_LAYOUT_BLOCK), warp per chunk, lane per (item, row
+// entity): the tet's block of that entity pair goes to one row pair (the row
+// entity's first-DoF row and its partner row, which hold the same tets). The
+// items of the chunk entity that hold the same row entity (the same position
+// byte) give the length of the row pair's list and the block's place in it, in
+// item order, so each output sums its contributions in the order of the packed
+// lists. Layout of the records: common.cuh.
 __global__ void __launch_bounds__(CC_WARPS * 32)
     k_chunk_blocks(const int32_t *ent_ptr, const Item *items, const uint32_t *ent_cnt, int64_t E, int64_t F,
-                   const int32_t *indptr, uint16_t *hoff, uint32_t *brec, int64_t *st) {
-  __shared__ int32_t cnt_all[CC_WARPS][CHUNK_MAX_POS / 2];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t chunk = (int64_t)blockIdx.x * CC_WARPS + w;
+                   const int32_t *indptr, uint32_t *brec, int64_t *st) {
+  struct Meta {
+    int32_t ptr[CHUNK + 1], c0[CHUNK + 1], ne[CHUNK], n_long;
+  };
+  __shared__ Meta meta[CC_WARPS];
+  const int lane = threadIdx.x & 31;
+  Meta &m = meta[threadIdx.x >> 5];
+  const int64_t chunk = (int64_t)blockIdx.x * CC_WARPS + (threadIdx.x >> 5);
   const int64_t nec = n_edge_chunks(E);
   if (chunk >= n_chunks(E, F)) return;
   const bool edges = chunk < nec;
   const int64_t x0 = edges ? chunk * CHUNK : E + (chunk - nec) * CHUNK;
   const int nx = (int)min((int64_t)CHUNK, (edges ? E : E + F) - x0);
   const int64_t cb0 = edges ? x0 : E + x0;
-  const int32_t my_ptr = lane <= nx ? ent_ptr[x0 + lane] : 0;
-  const int32_t my_c0 = lane <= nx ? indptr[cb0 + lane] : 0;
-  const uint32_t my_cnt = lane < nx ? ent_cnt[x0 + lane] : 0u;
-  const int32_t I0 = __shfl_sync(0xffffffffu, my_ptr, 0), I1 = __shfl_sync(0xffffffffu, my_ptr, nx);
-  const int32_t A0 = __shfl_sync(0xffffffffu, my_c0, 0), A0e = __shfl_sync(0xffffffffu, my_c0, nx);
-  const int Lsum = A0e - A0, Hsum = Lsum / 2;
-  if (Lsum > CHUNK_MAX_POS || I1 - I0 > CHUNK_MAX_ITEMS) {
+  if (lane <= nx) {
+    m.ptr[lane] = ent_ptr[x0 + lane];
+    m.c0[lane] = indptr[cb0 + lane];
+  }
+  if (lane < nx) m.ne[lane] = (int32_t)(ent_cnt[x0 + lane] & 0xffffu);
+  if (lane == 0) m.n_long = 0;
+  __syncwarp();
+  const int32_t I0 = m.ptr[0], nI = m.ptr[nx] - I0, A0 = m.c0[0];
+  const int Lsum = m.c0[nx] - A0, H = Lsum / 2;
+  if (Lsum > CHUNK_MAX_POS || nI > CHUNK_MAX_ITEMS) {
     if (lane == 0) flag(st, EMG_ST_CAPACITY, x0);
     return;
   }
-  const int64_t hb = (edges ? (int64_t)A0 : (int64_t)indptr[E] + (A0 - indptr[2 * E])) / 2;
-  int32_t *cnt = cnt_all[w];
-  for (int i = lane; i < Hsum; i += 32) cnt[i] = 0;
-  const int r = lane;  // row entity slot (0-5 edges, 6-9 faces) of the item's tet
-  __syncwarp();
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass == 1) {
-      int32_t carry = 0;
-      for (int b0 = 0; b0 < Hsum; b0 += 32) {
-        const int i = b0 + lane;
-        const int32_t v = i < Hsum ? cnt[i] : 0;
-        int32_t x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
-        }
-        if (i < Hsum) {
-          cnt[i] = carry + x - v;
-          hoff[hb + i] = (uint16_t)(carry + x - v);
-        }
-        carry += __shfl_sync(0xffffffffu, x, 31);
+  uint32_t *words = brec + (int64_t)kPairWords * I0;
+  uint2 *pairs = reinterpret_cast<uint2 *>(words);
+  const uint4 *raw = reinterpret_cast<const uint4 *>(items);
+  auto word_of = [&](const Item &rec, int r) {
+    const int s = rec.slot;
+    const int cb = s < 6 ? canon_dof(rec.ranks, s) : canon_dof(rec.ranks, 12 + (s - 6)) - 6;
+    const int ca = r < 6 ? canon_dof(rec.ranks, r) : canon_dof(rec.ranks, 12 + (r - 6)) - 6;
+    const int lo = ca < cb ? ca : cb, hi = ca < cb ? cb : ca;
+    return (uint32_t)((int64_t)rec.ia * 55 + block_index(lo, hi)) | (ca > cb ? 0x80000000u : 0u);
+  };
+  for (int t = lane; t < 10 * nI; t += 32) {
+    const int k = I0 + t / 10, r = t % 10;
+    int e = 0;
+    for (int q = 1; q < nx; ++q) e = k >= m.ptr[q] ? q : e;
+    const Item rec = items[k];
+    const uint32_t same = rec.pos[r] * 0x01010101u;
+    // bytes of an item: slot at 4, pos[0..9] at 5..14 (edges, then faces)
+    auto holds = [&](const uint4 &o) {
+      return r < 6 ? (__vcmpeq4(o.y, same) & 0xffffff00u) | (__vcmpeq4(o.z, same) & 0x00ffffffu)
+                   : (__vcmpeq4(o.z, same) & 0xff000000u) | (__vcmpeq4(o.w, same) & 0x00ffffffu);
+    };
+    const uint32_t word = word_of(rec, r);
+    int total = 0, rank = 0;
+    bool mixed = false;  // stored different ways round: only with inconsistent topology arrays
+    for (int i = m.ptr[e]; i < m.ptr[e + 1]; ++i)
+      if (holds(raw[i])) {
+        ++total;
+        rank += i < k ? 1 : 0;
+        if (i != k)
+          for (int p = r < 6 ? 0 : 6; p < (r < 6 ? 6 : 10); ++p)
+            if (items[i].pos[p] == rec.pos[r]) mixed = mixed || ((word_of(items[i], p) ^ word) >> 31);
       }
-      __syncwarp();
-    }
-    for (int32_t k = I0; k < I1; ++k) {
-      if (r < 10) {
-        int e = 0;
-        for (int q = 1; q < nx; ++q)
-          if (k >= __shfl_sync(0x3ffu, my_ptr, q)) e = q;
-        const int32_t ce = __shfl_sync(0x3ffu, my_c0, e);
-        const uint32_t c = __shfl_sync(0x3ffu, my_cnt, e);
-        const int ne = (int)(c & 0xffffu);
-        const Item rec = items[k];
-        const int h = (ce - A0) / 2 + (r < 6 ? 0 : ne) + rec.pos[r];
-        if (pass == 0) {
-          cnt[h] += 1;  // distinct h across the 10 lanes of one item
-        } else {
-          const int32_t at = cnt[h]++;
-          const int s = rec.slot;
-          const int cb = s < 6 ? canon_dof(rec.ranks, s) : canon_dof(rec.ranks, 12 + (s - 6)) - 6;
-          const int ca = r < 6 ? canon_dof(rec.ranks, r) : canon_dof(rec.ranks, 12 + (r - 6)) - 6;
-          const int lo = ca < cb ? ca : cb, hi = ca < cb ? cb : ca;
-          brec[(int64_t)10 * I0 + at] =
-              (uint32_t)((int64_t)rec.ia * 55 + block_index(lo, hi)) | (ca > cb ? 0x80000000u : 0u);
+    const int h = (m.c0[e] - A0) / 2 + (r < 6 ? 0 : m.ne[e]) + rec.pos[r];
+    const bool self = r == rec.slot;  // the entity's pair with itself: every item has one
+    if (self) words[2 * H + (k - I0)] = word;
+    if (total <= 2 && !mixed) {
+      if (total == 1) pairs[h] = make_uint2(word, kBlockNone);
+      else words[2 * h + rank] = word;
+    } else if (rank == 0) {  // one lane writes the whole list
+      int off = 0;
+      if (!self) {
+        off = 2 * H + nI + atomicAdd(&m.n_long, total);
+        uint32_t *list = words + off;
+        for (int i = m.ptr[e]; i < m.ptr[e + 1]; ++i) {
+          const Item o = items[i];
+          for (int p = r < 6 ? 0 : 6; p < (r < 6 ? 6 : 10); ++p)
+            if (o.pos[p] == rec.pos[r]) *list++ = word_of(o, p);
         }
       }
-      __syncwarp();
+      pairs[h] = make_uint2(self ? 0u : (uint32_t)off | ((uint32_t)total << 16), kBlockLong);
     }
   }
+}
+
+// chunk descriptors in processing order (common.cuh)
+__global__ void k_chunk_desc(const int32_t *ent_ptr, const Item *items, const uint32_t *ent_cnt, int64_t E, int64_t F,
+                             const int32_t *indptr, const int32_t *order, ChunkDesc *desc) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t nec = n_edge_chunks(E), nch = n_chunks(E, F);
+  if (g >= nch) return;
+  const int64_t chunk = order[g];
+  ChunkDesc d = {};
+  if (chunk >= 0 && chunk < nch) {
+    const bool edges = chunk < nec;
+    const int64_t x0 = edges ? chunk * CHUNK : E + (chunk - nec) * CHUNK;
+    const int nx = (int)min((int64_t)CHUNK, (edges ? E : E + F) - x0);
+    const int64_t cb0 = edges ? x0 : E + x0, cb1 = edges ? x0 + E : E + F + x0;
+    d.I0 = ent_ptr[x0];
+    d.A0 = indptr[cb0];
+    d.A1 = indptr[cb1];
+    d.faces = edges ? 0 : 1;
+    const int rows = indptr[cb0 + nx] - d.A0, n = ent_ptr[x0 + nx] - d.I0;
+    if (rows <= CHUNK_MAX_POS && n <= CHUNK_MAX_ITEMS) {  // else the build was flagged
+      d.H = (uint16_t)(rows / 2);
+      d.nI = (uint16_t)n;
+      for (int e = 0; e < CHUNK; ++e) {
+        d.hs[e] = d.H;
+        if (e >= nx) continue;
+        const int32_t i0 = ent_ptr[x0 + e], i1 = ent_ptr[x0 + e + 1];
+        d.hs[e] = (uint16_t)((indptr[cb0 + e] - d.A0) / 2);
+        d.ne[e] = (uint8_t)(ent_cnt[x0 + e] & 0xffu);
+        d.cnt[e] = (uint8_t)(i1 - i0);
+        if (i1 > i0) d.self[e] = items[i0].pos[items[i0].slot];
+      }
+    }
+  }
+  desc[g] = d;
+}
+
+int write_chunk_desc(const emg_plan *p, char *plan, const int32_t *indptr, cudaStream_t s) {
+  const int64_t nch = n_chunks(p->n_edges, p->n_tris);
+  k_chunk_desc<<<grid_for(nch, 128), 128, 0, s>>>(
+      reinterpret_cast<const int32_t *>(plan + p->off_ent_ptr), reinterpret_cast<const Item *>(plan + p->off_item),
+      reinterpret_cast<const uint32_t *>(plan + p->off_ent_cnt), p->n_edges, p->n_tris, indptr,
+      reinterpret_cast<const int32_t *>(plan + p->off_order), reinterpret_cast<ChunkDesc *>(plan + p->off_hoff));
+  return launch_check("k_chunk_desc");
 }
 
 __global__ void k_default_order(int32_t *order, int64_t nec, int64_t nch) {
@@ -582,9 +636,20 @@ __global__ void k_bitonic_step(uint64_t *keys, int64_t n2, int64_t j, int64_t k)
   }
 }
 
-__global__ void k_write_order(const uint64_t *keys, int64_t nch, int32_t *order) {
+// the new order; block layout: the chunk descriptors (by_chunk: in chunk
+// order) follow it
+__global__ void k_write_order(const uint64_t *keys, int64_t nch, int32_t *order, const ChunkDesc *by_chunk,
+                              ChunkDesc *desc) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < nch) order[g] = (int32_t)(keys[g] & 0xffffffffu);
+  if (g >= nch) return;
+  const int64_t c = (int64_t)(keys[g] & 0xffffffffu);
+  order[g] = (int32_t)c;
+  if (desc && c < nch) desc[g] = by_chunk[c];
+}
+
+__global__ void k_desc_by_chunk(const int32_t *order, const ChunkDesc *desc, int64_t nch, ChunkDesc *by_chunk) {
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g < nch && order[g] >= 0 && order[g] < nch) by_chunk[order[g]] = desc[g];
 }
 
 }  // namespace
@@ -617,14 +682,13 @@ size_t plan_layout(emg_plan *p) {
   p->off_posoff = o;
   o = align_up(o + (size_t)p->n_items * 20 * 2, 256);
   // per contribution the packed-layout indices of its two values (first- and
-  // second-DoF column), in the same order as contrib; block layout: one
-  // 4-byte block record per (item, row entity) and a uint16 list start per
-  // row pair (at most 10 per item)
+  // second-DoF column), in the same order as contrib; block layout: the row
+  // pairs' two-block records and the long lists, kPairWords words per item
   const bool block = p->value_layout == EMG_LAYOUT_BLOCK;
   p->off_pidx = o;
-  o = align_up(o + (size_t)p->n_items * (block ? 10 * 4 : 20 * (p->record_bytes == 4 ? 4 : 8)), 256);
-  p->off_hoff = o;
-  o = align_up(o + (block ? (size_t)p->n_items * 10 * 2 : 0), 256);
+  o = align_up(o + (size_t)p->n_items * (block ? kPairWords * 4 : 20 * (p->record_bytes == 4 ? 4 : 8)), 256);
+  p->off_hoff = o;  // block layout: the chunk descriptors
+  o = align_up(o + (block ? (size_t)n_chunks(p->n_edges, p->n_tris) * sizeof(ChunkDesc) : 0), 256);
   // the gather's chunk processing order
   p->off_order = o;
   o = align_up(o + (size_t)n_chunks(p->n_edges, p->n_tris) * 4, 256);
@@ -632,11 +696,16 @@ size_t plan_layout(emg_plan *p) {
   return o;
 }
 
-// chunk-order scratch: bounding-box partials and the sort keys (power of two)
+// chunk-order scratch: bounding-box partials, the sort keys (power of two) and
+// the chunk descriptors
 constexpr int BBOX_BLOCKS = 296;
+static size_t order_desc_offset(const emg_plan *p) {
+  return align_up(align_up((size_t)BBOX_BLOCKS * 6 * 8 + 64, 256) +
+                      (size_t)pow2_at_least(n_chunks(p->n_edges, p->n_tris)) * 8,
+                  256);
+}
 static size_t order_workspace_bytes(const emg_plan *p) {
-  return align_up((size_t)BBOX_BLOCKS * 6 * 8 + 64, 256) +
-         (size_t)pow2_at_least(n_chunks(p->n_edges, p->n_tris)) * 8;
+  return order_desc_offset(p) + (size_t)n_chunks(p->n_edges, p->n_tris) * sizeof(ChunkDesc);
 }
 
 // workspace: per-entity counters, per-column lengths, scan block sums, max
@@ -719,7 +788,9 @@ int plan_finish(const emg_plan *p, const int32_t *d_t2e, const int32_t *d_t2t, c
     const int rc = launch_check("k_default_order");
     if (rc) return rc;
   }
-  if (p->n_ent == 0 || p->n_assy == 0) return EMG_OK;
+  if (p->n_ent == 0) return EMG_OK;
+  if (p->n_assy == 0)  // empty columns; the block gather still walks the chunks
+    return p->value_layout == EMG_LAYOUT_BLOCK ? write_chunk_desc(p, plan, d_indptr, s) : EMG_OK;
   const int32_t *ent_ptr = reinterpret_cast<const int32_t *>(plan + p->off_ent_ptr);
   Item *items = reinterpret_cast<Item *>(plan + p->off_item);
   uint32_t *ent_cnt = reinterpret_cast<uint32_t *>(plan + p->off_ent_cnt);
@@ -741,9 +812,9 @@ int plan_finish(const emg_plan *p, const int32_t *d_t2e, const int32_t *d_t2t, c
   if ((rc = launch_check("k_chunk_contrib"))) return rc;
   if (!block) return EMG_OK;
   k_chunk_blocks<<<grid_for(n_chunks(p->n_edges, p->n_tris), CC_WARPS), CC_WARPS * 32, 0, s>>>(
-      ent_ptr, items, ent_cnt, p->n_edges, p->n_tris, d_indptr, reinterpret_cast<uint16_t *>(plan + p->off_hoff),
-      static_cast<uint32_t *>(pidx), d_status);
-  return launch_check("k_chunk_blocks");
+      ent_ptr, items, ent_cnt, p->n_edges, p->n_tris, d_indptr, static_cast<uint32_t *>(pidx), d_status);
+  if ((rc = launch_check("k_chunk_blocks"))) return rc;
+  return write_chunk_desc(p, plan, d_indptr, s);
 }
 
 int sort_u64(uint64_t *keys, int64_t n2, cudaStream_t s) {
@@ -777,7 +848,14 @@ int plan_order(const emg_plan *p, void *d_plan, const double *nodes, int64_t nN,
       nodes, nN, tets, p->n_tets, tetids, p->n_assy, box, p->n_edges, p->n_tris, nch, n2, keys);
   if ((rc = launch_check("k_chunk_keys"))) return rc;
   if ((rc = sort_u64(keys, n2, s))) return rc;
-  k_write_order<<<grid_for(nch, 256), 256, 0, s>>>(keys, nch, reinterpret_cast<int32_t *>(plan + p->off_order));
+  int32_t *order = reinterpret_cast<int32_t *>(plan + p->off_order);
+  ChunkDesc *by_chunk = reinterpret_cast<ChunkDesc *>(ws + order_desc_offset(p)), *desc = nullptr;
+  if (p->value_layout == EMG_LAYOUT_BLOCK) {
+    desc = reinterpret_cast<ChunkDesc *>(plan + p->off_hoff);
+    k_desc_by_chunk<<<grid_for(nch, 256), 256, 0, s>>>(order, desc, nch, by_chunk);
+    if ((rc = launch_check("k_desc_by_chunk"))) return rc;
+  }
+  k_write_order<<<grid_for(nch, 256), 256, 0, s>>>(keys, nch, order, by_chunk, desc);
   return launch_check("k_write_order");
 }
 

@@ -135,7 +135,7 @@ typedef struct {
   int32_t record_bytes;   /* 8 (default) or 4: bytes per contribution record of the packed gather */
   int32_t value_layout;   /* EMG_LAYOUT_PACKED (default) or EMG_LAYOUT_BLOCK: the element values
                              emg_assemble writes and its gather reads */
-  size_t off_hoff;        /* block layout: uint16 list start per row pair of every chunk */
+  size_t off_hoff;        /* block layout: 64-byte chunk descriptors, in processing order */
 } emg_plan;
 
 int emg_version(void);
@@ -175,9 +175,9 @@ int emg_plan_set_record_width(emg_plan *plan, int bytes);
  * layout of emg_assemble and of the plan's gather lists. EMG_LAYOUT_PACKED
  * (default): the canonical upper triangle, one record per (row, column pair)
  * contribution (record_bytes wide). EMG_LAYOUT_BLOCK: entity-pair blocks, one
- * 4-byte record per (row pair, column pair) contribution -- the two rows and
- * two columns of an entity pair come from the same tets, so one record and
- * one contiguous read give four entries of A. A is bit for bit the same in
+ * 8-byte record per (row pair, column pair) with the blocks of its tets -- the
+ * two rows and two columns of an entity pair come from the same tets, so one
+ * record and one contiguous read per tet give four entries of A. A is bit for bit the same in
  * both layouts. Updates plan_bytes. No counterpart in the reference. */
 int emg_plan_set_value_layout(emg_plan *plan, int layout);
 
