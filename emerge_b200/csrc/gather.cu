@@ -55,13 +55,13 @@ __device__ __forceinline__ C64 load_val(const void *p, int64_t idx) {
   }
 }
 
-// Pull gather (every layout). A warp owns one entity chunk (CHUNK consecutive
-// entities of one kind, see common.cuh); its two output runs are contiguous.
-// Lane l owns positions l, l+32, ... of the runs: it reads the position's
-// contribution list from the plan (item of the chunk, element row), sums the
-// contributing element values in that fixed order (items ascending, so tets
-// ascending), and writes the first-DoF and second-DoF entries once. No shared
-// memory, no atomics; each nonzero is produced by exactly one lane.
+// Packed gather. A warp owns one entity chunk (CHUNK consecutive entities of one
+// kind, see common.cuh); its two output runs are contiguous. Lane l owns
+// positions l, l+32, ... of the runs: it reads the position's contribution list
+// from the plan, sums the contributing element values in that fixed order (items
+// ascending, so tets ascending), and writes the first-DoF and second-DoF entries
+// once. No shared memory, no atomics; each nonzero is produced by exactly one
+// lane.
 constexpr int PG_WARPS = 8;
 
 // element slots (row r, column a0) and (row r, column a1) of the reference COO
@@ -119,44 +119,73 @@ __device__ __forceinline__ bool chunk_meta(const int32_t *ent_ptr, const int32_t
   return true;
 }
 
-// reference COO layout (any COO data of this field's slot layout)
+// Reference COO layout (any COO data of this field's slot layout), a warp per
+// entity: its two columns are summed in shared memory, item by item in the
+// plan's order, so that each entry adds its contributions in the order of the
+// other layouts; the plan holds no lists for it. The 20 rows of an item's tet are
+// 20 different rows of the column, one lane each, and the values of COO_ITEMS
+// items are in flight.
+constexpr int COO_ITEMS = 4;
+
 template <typename R, bool TWO>
-__global__ void __launch_bounds__(PG_WARPS * 32)
-    k_gather_coo(const int32_t *ent_ptr, const int32_t *order, const Item *items, const uint16_t *contrib,
-                 const uint16_t *posoff, int64_t E, int64_t F, const int32_t *indptr, const void *v1, const void *v2, double ar, double ai,
-                 double br, double bi, double2 *A) {
-  const int lane = threadIdx.x & 31;
-  ChunkMeta m;
-  if (!chunk_meta(ent_ptr, order, indptr, E, F, (int64_t)blockIdx.x * PG_WARPS + (threadIdx.x >> 5), m)) return;
-  const int total = 20 * (m.I1 - m.I0);
-  const uint16_t *clist = contrib + (int64_t)20 * m.I0;
-  const Item *it = items + m.I0;
-  for (int p = lane; p < m.Lsum; p += 32) {
-    const int o0 = posoff[m.hbase + p];
-    const int o1 = min(p + 1 < m.Lsum ? (int)posoff[m.hbase + p + 1] : total, total);
-    double s0r = 0.0, s0i = 0.0, s1r = 0.0, s1i = 0.0;
-    for (int k = o0; k < o1; ++k) {
-      const uint32_t c = clist[k];
-      if ((int)(c >> 5) >= m.I1 - m.I0) continue;  // only a plan whose build was flagged can hold this
-      const uint4 rec = __ldg(reinterpret_cast<const uint4 *>(it + (c >> 5)));
-      const int r = (int)(c & 31u);
-      C64 u0, u1;
-      load_coo_pair<R>(v1, (int)rec.x, (int)(rec.y & 0xffu), r, u0, u1);
-      s0r += ar * u0.re - ai * u0.im;
-      s0i += ar * u0.im + ai * u0.re;
-      s1r += ar * u1.re - ai * u1.im;
-      s1i += ar * u1.im + ai * u1.re;
-      if (TWO) {
-        C64 t0, t1;
-        load_coo_pair<R>(v2, (int)rec.x, (int)(rec.y & 0xffu), r, t0, t1);
-        s0r += br * t0.re - bi * t0.im;
-        s0i += br * t0.im + bi * t0.re;
-        s1r += br * t1.re - bi * t1.im;
-        s1i += br * t1.im + bi * t1.re;
-      }
+__global__ void k_gather_coo(const int32_t *ent_ptr, const int32_t *order, const Item *items, const uint32_t *ent_cnt,
+                             int64_t E, int64_t F, const int32_t *indptr, const void *v1, const void *v2, double ar,
+                             double ai, double br, double bi, int max_col, double2 *A) {
+  extern __shared__ __align__(16) double2 coo_cols[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
+  const int64_t nec = n_edge_chunks(E), nch = n_chunks(E, F);
+  if (g >= nch * CHUNK) return;
+  const int64_t chunk = __ldg(order + g / CHUNK);
+  if (chunk < 0 || chunk >= nch) return;  // only a corrupted plan can hold this
+  const bool edges = chunk < nec;
+  const int64_t x = (edges ? chunk * CHUNK : E + (chunk - nec) * CHUNK) + g % CHUNK;
+  if (x >= (edges ? E : E + F)) return;
+  const int64_t c0 = edges ? x : E + x, c1 = edges ? x + E : E + F + x;
+  const int64_t A0 = indptr[c0], A1 = indptr[c1];
+  const int rows = (int)(indptr[c0 + 1] - A0);
+  if (rows > max_col) return;  // as above
+  const uint32_t cnt = ent_cnt[x];
+  const int ne = (int)(cnt & 0xffffu), nf = (int)(cnt >> 16);
+  double2 *s0 = coo_cols + (int64_t)w * 2 * max_col, *s1 = s0 + max_col;
+  for (int i = lane; i < rows; i += 32) s0[i] = s1[i] = make_double2(0.0, 0.0);
+  __syncwarp();
+  const int r = lane;  // row slot of the tet
+  const int slot = r < 6 ? r : (r < 12 ? r - 6 : (r < 16 ? r - 6 : r - 10));
+  const int off = r < 6 ? 0 : (r < 12 ? ne : (r < 16 ? 2 * ne : 2 * ne + nf));
+  const int b = ent_ptr[x], e = ent_ptr[x + 1];
+  for (int k0 = b; k0 < e; k0 += COO_ITEMS) {
+    C64 u[COO_ITEMS][2], t[COO_ITEMS][2];
+    int at[COO_ITEMS];
+#pragma unroll
+    for (int k = 0; k < COO_ITEMS; ++k) {
+      at[k] = -1;
+      if (k0 + k >= e || r >= 20) continue;
+      const Item rec = items[k0 + k];
+      at[k] = off + rec.pos[slot];
+      load_coo_pair<R>(v1, rec.ia, rec.slot, r, u[k][0], u[k][1]);
+      if (TWO) load_coo_pair<R>(v2, rec.ia, rec.slot, r, t[k][0], t[k][1]);
     }
-    A[m.A0 + p] = make_double2(s0r, s0i);
-    A[m.A1 + p] = make_double2(s1r, s1i);
+#pragma unroll
+    for (int k = 0; k < COO_ITEMS; ++k) {
+      if (at[k] >= 0 && at[k] < rows)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          double2 s = (c ? s1 : s0)[at[k]];
+          s.x += ar * u[k][c].re - ai * u[k][c].im;
+          s.y += ar * u[k][c].im + ai * u[k][c].re;
+          if (TWO) {
+            s.x += br * t[k][c].re - bi * t[k][c].im;
+            s.y += br * t[k][c].im + bi * t[k][c].re;
+          }
+          (c ? s1 : s0)[at[k]] = s;
+        }
+      __syncwarp();
+    }
+  }
+  for (int i = lane; i < rows; i += 32) {
+    A[A0 + i] = s0[i];
+    A[A1 + i] = s1[i];
   }
 }
 
@@ -573,9 +602,7 @@ int launch_gather(const emg_plan *p, const void *d_plan, const int32_t *d_indptr
   const int32_t *ent_ptr = reinterpret_cast<const int32_t *>(plan + p->off_ent_ptr);
   const Item *items = reinterpret_cast<const Item *>(plan + p->off_item);
   const int32_t *order = reinterpret_cast<const int32_t *>(plan + p->off_order);
-  const uint16_t *contrib = reinterpret_cast<const uint16_t *>(plan + p->off_contrib);
   const uint16_t *posoff = reinterpret_cast<const uint16_t *>(plan + p->off_posoff);
-  const int g = grid_for(n_chunks(p->n_edges, p->n_tris), PG_WARPS);
   double2 *A = static_cast<double2 *>(d_A);
   const bool two = d_v2 != nullptr;
   const bool f32 = values_fp32(precision);
@@ -612,9 +639,15 @@ int launch_gather(const emg_plan *p, const void *d_plan, const int32_t *d_indptr
 #undef EMG_PK
     return launch_check("k_gather_packed");
   }
-#define EMG_COO(R, TWO)                                                                                           \
-  k_gather_coo<R, TWO><<<g, PG_WARPS * 32, 0, s>>>(ent_ptr, order, items, contrib, posoff, p->n_edges, p->n_tris, \
-                                                   d_indptr, d_v1, d_v2, ar, ai, br, bi, A)
+  // two columns per warp, at most four warps and 48 KB per CTA
+  const uint32_t *ent_cnt = reinterpret_cast<const uint32_t *>(plan + p->off_ent_cnt);
+  const int max_col = p->max_col > 0 && p->max_col < 1536 ? (int)p->max_col : 1536;
+  const int warps = std::max(1, std::min(4, (48 << 10) / (32 * max_col)));
+  const int g = grid_for(n_chunks(p->n_edges, p->n_tris) * CHUNK, warps);
+#define EMG_COO(R, TWO)                                                                                             \
+  k_gather_coo<R, TWO><<<g, warps * 32, 32 * max_col * warps, s>>>(ent_ptr, order, items, ent_cnt, p->n_edges,       \
+                                                                   p->n_tris, d_indptr, d_v1, d_v2, ar, ai, br, bi, \
+                                                                   max_col, A)
   if (f32) {
     if (two) EMG_COO(float, true); else EMG_COO(float, false);
   } else {

@@ -305,7 +305,7 @@ __global__ void k_max_col(const int32_t *col_len, int64_t n, int32_t *out) {
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-// Gather lists, warp per chunk: every (item, row) of the chunk contributes to
+// Packed gather lists, warp per chunk: every (item, row) of the chunk contributes to
 // one position of the chunk's first-DoF run (and the same position of its
 // second-DoF run). Count per position, scan, then place the contributions in
 // item order (items of an entity are sorted by tet), so each output sums its
@@ -314,8 +314,7 @@ constexpr int CC_WARPS = 8;
 
 __global__ void __launch_bounds__(CC_WARPS * 32)
     k_chunk_contrib(const int32_t *ent_ptr, const Item *items, const uint32_t *ent_cnt, int64_t E, int64_t F,
-                    const int32_t *indptr, uint16_t *contrib, uint16_t *posoff, void *pidx_v, bool compact,
-                    int64_t *st) {
+                    const int32_t *indptr, uint16_t *posoff, void *pidx_v, bool compact, int64_t *st) {
   __shared__ int32_t cnt_all[CC_WARPS][CHUNK_MAX_POS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t chunk = (int64_t)blockIdx.x * CC_WARPS + w;
@@ -378,16 +377,15 @@ __global__ void __launch_bounds__(CC_WARPS * 32)
           cnt[p] += 1;  // distinct p across the 20 lanes of one item
         } else {
           const int32_t at = cnt[p]++;
-          contrib[(int64_t)20 * I0 + at] = (uint16_t)(((k - I0) << 5) | r);
           const int s = rec.slot;
           const int a0 = s < 6 ? s : 12 + (s - 6), a1 = s < 6 ? s + 6 : 16 + (s - 6);
           const int al = canon_dof(rec.ranks, r);
           const int b0 = canon_dof(rec.ranks, a0), b1 = canon_dof(rec.ranks, a1);
           const int64_t base = (int64_t)rec.ia * 210;
-          if (pidx_v && compact)
+          if (compact)
             static_cast<uint32_t *>(pidx_v)[(int64_t)20 * I0 + at] =
                 (uint32_t)(base + packed_index(min(al, b0), max(al, b0))) | (al <= b0 ? 0x80000000u : 0u);
-          else if (pidx_v)
+          else
             static_cast<int2 *>(pidx_v)[(int64_t)20 * I0 + at] =
                 make_int2((int)(base + packed_index(min(al, b0), max(al, b0))),
                           (int)(base + packed_index(min(al, b1), max(al, b1))));
@@ -673,18 +671,15 @@ size_t plan_layout(emg_plan *p) {
   p->off_item_pos = p->off_item;  // positions live inside the item records
   p->off_ent_cnt = o;
   o = align_up(o + (size_t)p->n_ent * 4, 256);
-  // 20 contributions (uint16: item-in-chunk << 5 | row) per item, and one
-  // uint16 start offset per first-DoF output position; a column of entity x
-  // has 2 (n_adj_edges + n_adj_faces) <= 20 * items(x) entries, so 20 per item
-  // bounds the positions before nnz is known
-  p->off_contrib = o;
-  o = align_up(o + (size_t)p->n_items * 20 * 2, 256);
-  p->off_posoff = o;
-  o = align_up(o + (size_t)p->n_items * 20 * 2, 256);
-  // per contribution the packed-layout indices of its two values (first- and
-  // second-DoF column), in the same order as contrib; block layout: the row
-  // pairs' two-block records and the long lists, kPairWords words per item
+  // packed layout: one uint16 list start per first-DoF output position; a column
+  // of entity x has 2 (n_adj_edges + n_adj_faces) <= 20 * items(x) entries, so 20
+  // per item bounds the positions before nnz is known
   const bool block = p->value_layout == EMG_LAYOUT_BLOCK;
+  p->off_contrib = p->off_posoff = o;
+  o = align_up(o + (block ? 0 : (size_t)p->n_items * 20 * 2), 256);
+  // packed layout: per contribution the indices of its two values (first- and
+  // second-DoF column); block layout: the row
+  // pairs' two-block records and the long lists, kPairWords words per item
   p->off_pidx = o;
   o = align_up(o + (size_t)p->n_items * (block ? kPairWords * 4 : 20 * (p->record_bytes == 4 ? 4 : 8)), 256);
   p->off_hoff = o;  // block layout: the chunk descriptors
@@ -799,18 +794,13 @@ int plan_finish(const emg_plan *p, const int32_t *d_t2e, const int32_t *d_t2t, c
       d_indptr, d_indices, d_status);
   int rc = launch_check("k_entity_rows<fill>");
   if (rc) return rc;
-  uint16_t *contrib = reinterpret_cast<uint16_t *>(plan + p->off_contrib);
-  uint16_t *posoff = reinterpret_cast<uint16_t *>(plan + p->off_posoff);
   void *pidx = plan + p->off_pidx;
-  const bool compact = p->record_bytes == 4;
-  const bool block = p->value_layout == EMG_LAYOUT_BLOCK;
-  // the block layout keeps the (item, row) lists for the COO gather and puts
-  // its own records where the packed records would be
-  k_chunk_contrib<<<grid_for(n_chunks(p->n_edges, p->n_tris), CC_WARPS), CC_WARPS * 32, 0, s>>>(
-      ent_ptr, items, ent_cnt, p->n_edges, p->n_tris, d_indptr, contrib, posoff, block ? nullptr : pidx, compact,
-      d_status);
-  if ((rc = launch_check("k_chunk_contrib"))) return rc;
-  if (!block) return EMG_OK;
+  if (p->value_layout != EMG_LAYOUT_BLOCK) {
+    k_chunk_contrib<<<grid_for(n_chunks(p->n_edges, p->n_tris), CC_WARPS), CC_WARPS * 32, 0, s>>>(
+        ent_ptr, items, ent_cnt, p->n_edges, p->n_tris, d_indptr, reinterpret_cast<uint16_t *>(plan + p->off_posoff),
+        pidx, p->record_bytes == 4, d_status);
+    return launch_check("k_chunk_contrib");
+  }
   k_chunk_blocks<<<grid_for(n_chunks(p->n_edges, p->n_tris), CC_WARPS), CC_WARPS * 32, 0, s>>>(
       ent_ptr, items, ent_cnt, p->n_edges, p->n_tris, d_indptr, static_cast<uint32_t *>(pidx), d_status);
   if ((rc = launch_check("k_chunk_blocks"))) return rc;

@@ -126,9 +126,10 @@ typedef struct {
   int64_t nnz;       /* set by emg_plan_build */
   int64_t max_col;   /* longest column, set by emg_plan_build */
   size_t off_ent_ptr, off_item, off_item_pos, off_ent_cnt; /* byte offsets in the blob */
-  size_t off_contrib, off_posoff, off_pidx; /* gather lists: per output position of
-                                     every entity chunk, its contributions as
-                                     (item, row) and as packed value indices */
+  size_t off_contrib, off_posoff, off_pidx; /* packed layout: per output position of
+                                     every entity chunk its list start (posoff,
+                                     contrib the same) and the list's value indices;
+                                     block layout: the row pairs' block records (pidx) */
   size_t off_order;       /* int32 per entity chunk: the gather's processing order */
   size_t plan_bytes;      /* blob size */
   size_t workspace_bytes; /* scratch needed by emg_plan_build and emg_plan_order */
