@@ -289,6 +289,7 @@ int emg_assemble_batch(const emg_assembly_job *h_jobs, int n_jobs, int precision
   int64_t *gcta = reinterpret_cast<int64_t *>(h + batch_offset(n_jobs, 3));
   const int kind = h_jobs[0].mat.kind;
   const int layout = h_jobs[0].plan ? h_jobs[0].plan->value_layout : EMG_LAYOUT_PACKED;
+  const int tets_per_cta = elem_tets_per_cta(precision, kind);
   ecta[0] = gcta[0] = 0;
   bool wide = true;
   for (int i = 0; i < n_jobs; ++i) {
@@ -303,7 +304,7 @@ int emg_assemble_batch(const emg_assembly_job *h_jobs, int n_jobs, int precision
     if (p->n_assy < p->n_tets && !j.d_tetids) return fail(EMG_EINVAL, "job %d: tetids required", i);
     ea[i] = ElemArgs{j.d_nodes, j.n_nodes, j.d_tets, p->n_tets, j.d_tetids, p->n_assy, j.mat.d_er, j.mat.d_ur,
                      j.alpha_re, j.alpha_im, j.beta_re, j.beta_im, j.d_values, j.d_status};
-    ecta[i + 1] = ecta[i] + (p->n_assy + 127) / 128;
+    ecta[i + 1] = ecta[i] + (p->n_assy + tets_per_cta - 1) / tets_per_cta;
     int rc = gather_job_fill(p, j.d_plan, j.d_indptr, j.d_values, j.d_A, precision, &ga[i]);
     if (rc) return rc;
     gcta[i + 1] = gcta[i] + (p->n_ent > 0 ? ga[i].n_ctas : 0);

@@ -205,6 +205,12 @@ inline int persistent_ctas(int per_sm) {
   return (sms[dev] > 0 ? sms[dev] : 148) * per_sm;
 }
 
+// tets of one CTA of the element kernel, by precision (EMG_FP64, ...) and
+// material kind: 128 threads, two of them per tet for complex tensors in FP64
+constexpr int elem_tets_per_cta(int precision, int kind) {
+  return kind != EMG_MAT_ISO && precision != EMG_MIXED ? 64 : 128;
+}
+
 // element kernel launchers, one translation unit per (form, material kind);
 // form 0 = reference-faithful FP64, 1 = mixed, 2 = exact closed form
 #define EMG_DECLARE_ELEM(F, K) int launch_element_##F##_##K(const ElemArgs &a, int layout, cudaStream_t s);

@@ -35,6 +35,23 @@ namespace emg {
 namespace {
 
 enum { FORM_REF64 = 0, FORM_REF32 = 1, FORM_EXACT = 2 };
+
+// Complex tensors in FP64 (diagonal and full materials, both FP64 forms): two
+// lanes share a tet, the even one computes the real parts of its values, the
+// odd one the imaginary parts. With alpha and beta multiplied into the tensors
+// first, each part is a real contraction, half the tensor registers of a complex
+// one, and the lanes share the quadrature points (REF64). A lane per tet spilled
+// 1.1 KB (diagonal) and 6.9 KB (full). Measured: diagonal at 1,008,000 tets 2,447
+// -> 1,110 us (EXACT 726 -> 660), full at 414,720 1,856 -> 555 (1,276 -> 361).
+// Bound: FP64 latency at eight warps per SM (254 registers).
+// Full tensors go through their symmetric halves first (all there is to a
+// reciprocal material); a warp that has any other adds the antisymmetric halves'
+// part in a second pass (both halves in one pass kept 4.9 KB spilled: 1,607 us).
+enum { KIND_PAIR = 3, KIND_PAIR_FULL = 4, KIND_PAIR_ANTI = 5 };
+__host__ __device__ constexpr int tensor_kind(int form, int kind) {
+  return form == FORM_REF32 || kind == EMG_MAT_ISO ? kind : (kind == EMG_MAT_DIAG ? KIND_PAIR : KIND_PAIR_FULL);
+}
+__host__ __device__ constexpr int lanes_per_tet(int tensor_kind) { return tensor_kind >= KIND_PAIR ? 2 : 1; }
 template <int FORM>
 struct FormReal {
   using T = double;
@@ -281,9 +298,10 @@ namespace {
 constexpr int NMOM = emg_mtables::kNumMoments;
 
 // Reference forms: coefficients, quadrature points and L~ exactly as the
-// reference computes them, then the quadrature moments. Returns false for a
-// degenerate tet.
-template <typename R>
+// reference computes them, then the quadrature moments: of all 11 points, or
+// (PAIR) of this lane's half of them, the even lane's the first six. Returns
+// false for a degenerate tet.
+template <bool PAIR, typename R>
 __device__ __forceinline__ bool ref_geometry(const double X[3][4], const int64_t v[4], Geo &G, R mu[NMOM]) {
   int rank[4];
   uint64_t inv;
@@ -301,7 +319,8 @@ __device__ __forceinline__ bool ref_geometry(const double X[3][4], const int64_t
     c[q] = cc[q] / six_v;
     d[q] = cd[q] / six_v;
   }
-  double br[4], cr[4], dr[4];
+  double Ar[4], br[4], cr[4], dr[4];
+  scatter_rank(a, rank, Ar);
   scatter_rank(b, rank, br);
   scatter_rank(c, rank, cr);
   scatter_rank(d, rank, dr);
@@ -314,25 +333,22 @@ __device__ __forceinline__ bool ref_geometry(const double X[3][4], const int64_t
   G.V = V;
   G.sig = 1.0;
   G.inv = inv;
-#pragma unroll
-  for (int i = 0; i < NMOM; ++i) mu[i] = (R)0;
   // rolled on purpose: the kernel is instruction-fetch bound, and the point
   // loop body is the same for all 11 points
 #pragma unroll 1
-  for (int q = 0; q < 11; ++q) {
+  for (int i = 0; i < (PAIR ? 6 : 11); ++i) {
+    const int q = PAIR ? min(((threadIdx.x & 1) ? 6 : 0) + i, 10) : i;
+    const double w = PAIR && (threadIdx.x & 1) && i == 5 ? 0.0 : kDP[0][q];  // the odd lane has five points
     const double p1 = kDP[1][q], p2 = kDP[2][q], p3 = kDP[3][q], p4 = kDP[4][q];
     double xq[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k)
       xq[k] = EMG_A(EMG_A(EMG_A(EMG_M2(X[k][0], p1), EMG_M2(X[k][1], p2)), EMG_M2(X[k][2], p3)), EMG_M2(X[k][3], p4));
-    double L[4];
+    R Lq[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m)
-      L[m] = EMG_A(EMG_A(EMG_A(a[m], EMG_M2(b[m], xq[0])), EMG_M2(c[m], xq[1])), EMG_M2(d[m], xq[2]));
-    double Lr[4];
-    scatter_rank(L, rank, Lr);
-    R Lq[4] = {(R)Lr[0], (R)Lr[1], (R)Lr[2], (R)Lr[3]};
-    emg_mtables::emg_moments<R>(Lq, (R)kDP[0][q], mu);
+    for (int r = 0; r < 4; ++r)
+      Lq[r] = (R)EMG_A(EMG_A(EMG_A(Ar[r], EMG_M2(br[r], xq[0])), EMG_M2(cr[r], xq[1])), EMG_M2(dr[r], xq[2]));
+    emg_mtables::emg_moments<R>(Lq, (R)w, mu);
   }
   return true;
 }
@@ -393,6 +409,19 @@ struct Tensors {
 };
 template <typename R>
 struct Tensors<EMG_MAT_ISO, R> {
+  R G[4][4], H[6][6];
+};
+// the lane's part (real or imaginary) of beta G and alpha H
+template <typename R>
+struct Tensors<KIND_PAIR, R> {
+  R G[4][4], H[6][6];
+};
+template <typename R>
+struct Tensors<KIND_PAIR_FULL, R> {
+  R G[4][4], H[6][6];
+};
+template <typename R>
+struct Tensors<KIND_PAIR_ANTI, R> {
   R G[4][4], H[6][6];
 };
 
@@ -473,9 +502,66 @@ __device__ __forceinline__ void build_cplx(const Geo &Gm, const C64 eps[9], cons
     }
 }
 
+// The lane's part of the forms V b . t a of a 3x3 tensor t (row-major): (e g_m).g_n
+// into G and (u X_P).X_Q into H, of the tensors' symmetric or antisymmetric halves.
+template <int KIND, typename R>
+__device__ __forceinline__ void build_pair(const Geo &Gm, const double e[9], const double u[9], Tensors<KIND, R> &T) {
+  double X[6][3];
+  const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
+#pragma unroll
+  for (int p = 0; p < 6; ++p) cross3(Gm.g[pa[p]], Gm.g[pb[p]], X[p]);
+  auto form = [&](const double t[9], const double a[3], const double b[3]) {
+    double s = 0.0;
+    if constexpr (KIND == KIND_PAIR_ANTI) {  // b . t a = w . (a x b), w = (t21, t02, t10)
+      double c[3];
+      cross3(a, b, c);
+      s = 0.5 * ((t[7] - t[5]) * c[0] + (t[2] - t[6]) * c[1] + (t[3] - t[1]) * c[2]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (KIND == KIND_PAIR && r != c) continue;
+          const double v = r == c ? t[4 * r] : 0.5 * (t[3 * r + c] + t[3 * c + r]);
+          s += v * (b[r] * a[c]);
+        }
+    }
+    return s * Gm.V;
+  };
+  constexpr bool anti = KIND == KIND_PAIR_ANTI;
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n = m; n < 4; ++n) {
+      const R v = anti && n == m ? (R)0 : (R)form(e, Gm.g[m], Gm.g[n]);
+      T.G[n][m] = anti ? -v : v;
+      T.G[m][n] = v;
+    }
+#pragma unroll
+  for (int p = 0; p < 6; ++p)
+#pragma unroll
+    for (int q = p; q < 6; ++q) {
+      const R v = anti && q == p ? (R)0 : (R)form(u, X[p], X[q]);
+      T.H[q][p] = anti ? -v : v;
+      T.H[p][q] = v;
+    }
+}
+
 template <int KIND, typename R>
 struct EntryT {
   using T = CR<R>;
+};
+template <typename R>
+struct EntryT<KIND_PAIR, R> {
+  using T = R;
+};
+template <typename R>
+struct EntryT<KIND_PAIR_FULL, R> {
+  using T = R;
+};
+template <typename R>
+struct EntryT<KIND_PAIR_ANTI, R> {
+  using T = R;
 };
 template <typename R>
 struct EntryT<EMG_MAT_ISO, R> {
@@ -514,6 +600,16 @@ __device__ __forceinline__ void entry(const Tensors<KIND, R> &T, const R *mu, do
   m = am;
 }
 
+// The lane's part of entry (lo, hi). Antisymmetric half: the first function is
+// the DoF with the lower reference index (curlcurl.py:358-376).
+template <int lo, int hi, int FORM, int KIND, typename R>
+__device__ __forceinline__ R pair_value(const Tensors<KIND, R> &T, const R *mu, double sig, uint64_t inv) {
+  R k, m;
+  entry<lo, hi, FORM, KIND, R>(T, mu, sig, k, m);
+  if (KIND == KIND_PAIR_ANTI && ref_dof(inv, lo) > ref_dof(inv, hi)) return -(k + m);
+  return k + m;
+}
+
 template <typename R>
 struct StoreT;
 template <>
@@ -526,28 +622,42 @@ struct StoreT<float> {
 };
 
 constexpr int ELEM_THREADS = 128;
-constexpr int ELEM_WARPS = ELEM_THREADS / 32;
 
 __device__ __forceinline__ double cfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float cfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double cmul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float cmul_rn(float a, float b) { return __fmul_rn(a, b); }
 
+// a staged value into the output: the second pass of a full tensor adds to the first's
+template <int KIND, typename ST>
+__device__ __forceinline__ void put(ST *o, ST v) {
+  if (KIND == KIND_PAIR_ANTI) {
+    const ST was = *o;
+    v.x += was.x;
+    v.y += was.y;
+  }
+  *o = v;
+}
+
 template <int x, int y, int FORM, int KIND, typename R>
 __device__ __forceinline__ void compute_store(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
                                               const CR<R> &cM, uint64_t inv, int rx, typename StoreT<R>::T *row) {
   using ST = typename StoreT<R>::T;
+  constexpr int lo = x < y ? x : y, hi = x < y ? y : x;
   const int b = ref_dof(inv, y);
   ST v;
-  if constexpr (KIND == EMG_MAT_ISO) {
+  if constexpr (KIND >= KIND_PAIR) {
+    reinterpret_cast<R *>(row + b)[threadIdx.x & 1] = pair_value<lo, hi, FORM, KIND, R>(T, mu, sig, inv);
+    return;
+  } else if constexpr (KIND == EMG_MAT_ISO) {
     R k0, m0;
-    entry<(x < y ? x : y), (x < y ? y : x), FORM, KIND, R>(T, mu, sig, k0, m0);
+    entry<lo, hi, FORM, KIND, R>(T, mu, sig, k0, m0);
     v.x = cfma(cK.re, k0, cmul_rn(cM.re, m0));
     v.y = cfma(cK.im, k0, cmul_rn(cM.im, m0));
   } else {
     CR<R> k, m;
     if constexpr (KIND == EMG_MAT_DIAG) {
-      entry<(x < y ? x : y), (x < y ? y : x), FORM, KIND, R>(T, mu, sig, k, m);
+      entry<lo, hi, FORM, KIND, R>(T, mu, sig, k, m);
     } else {
       // first = the DoF with the lower reference index (curlcurl.py:358-376)
       if (rx <= b) {
@@ -573,21 +683,22 @@ template <int FORM, int KIND, typename R, int X>
 __device__ __forceinline__ void do_row(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
                                        const CR<R> &cM, uint64_t inv, bool active, int ia,
                                        typename StoreT<R>::T *stage, typename StoreT<R>::T *out) {
+  constexpr int LPT = lanes_per_tet(KIND);
   const int lane = threadIdx.x & 31;
   const int rx = ref_dof(inv, X);
   if (active)
-    compute_row<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, rx, stage + lane * 21,
+    compute_row<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, rx, stage + lane / LPT * 21,
                                   std::make_integer_sequence<int, 20>{});
   __syncwarp();
-  // cooperative, coalesced write of the warp's 32 rows (each 20 contiguous values)
+  // cooperative, coalesced write of the warp's rows (one of 20 contiguous values per tet)
 #pragma unroll 1
-  for (int it = 0; it < 20; ++it) {
+  for (int it = 0; it < 20 / LPT; ++it) {
     int e = it * 32 + lane;
     int r = e / 20, c = e - r * 20;
-    int ia_r = __shfl_sync(0xffffffffu, ia, r);
-    int a_r = __shfl_sync(0xffffffffu, rx, r);
-    bool act_r = __shfl_sync(0xffffffffu, (int)active, r);
-    if (act_r) out[(int64_t)ia_r * 400 + a_r * 20 + c] = stage[r * 21 + c];
+    int ia_r = __shfl_sync(0xffffffffu, ia, r * LPT);
+    int a_r = __shfl_sync(0xffffffffu, rx, r * LPT);
+    bool act_r = __shfl_sync(0xffffffffu, (int)active, r * LPT);
+    if (act_r) put<KIND>(out + (int64_t)ia_r * 400 + a_r * 20 + c, stage[r * 21 + c]);
   }
   __syncwarp();
 }
@@ -610,7 +721,10 @@ __device__ __forceinline__ void compute_store_packed(const Tensors<KIND, R> &T, 
                                                      typename StoreT<R>::T *row) {
   using ST = typename StoreT<R>::T;
   ST v;
-  if constexpr (KIND == EMG_MAT_ISO) {
+  if constexpr (KIND >= KIND_PAIR) {
+    reinterpret_cast<R *>(row + (y - x))[threadIdx.x & 1] = pair_value<x, y, FORM, KIND, R>(T, mu, sig, inv);
+    return;
+  } else if constexpr (KIND == EMG_MAT_ISO) {
     R k0, m0;
     entry<x, y, FORM, KIND, R>(T, mu, sig, k0, m0);
     v.x = cfma(cK.re, k0, cmul_rn(cM.re, m0));
@@ -644,20 +758,19 @@ template <int FORM, int KIND, typename R, int X>
 __device__ __forceinline__ void do_row_packed(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
                                               const CR<R> &cM, uint64_t inv, bool active, int ia,
                                               typename StoreT<R>::T *stage, typename StoreT<R>::T *out) {
-  constexpr int W = 20 - X;
+  constexpr int W = 20 - X, LPT = lanes_per_tet(KIND);
   const int lane = threadIdx.x & 31;
   if (active)
-    compute_row_packed<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane * (W | 1),
+    compute_row_packed<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane / LPT * (W | 1),
                                          std::make_integer_sequence<int, W>{});
-  // the warp's 32 tets are consecutive assembled indices: lane r's is ia - lane + r
+  // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
   const unsigned act = __ballot_sync(0xffffffffu, active);
-  const int64_t ia_w = (int64_t)ia - lane;
+  const int64_t ia_w = (int64_t)ia - lane / LPT;
   __syncwarp();
 #pragma unroll 2
-  for (int it = 0; it < W; ++it) {
-    const int e = it * 32 + lane;
+  for (int e = lane; e < 32 / LPT * W; e += 32) {
     const int r = e / W, c = e - r * W;
-    if ((act >> r) & 1u) out[(ia_w + r) * 210 + packed_index(X, X) + c] = stage[r * (W | 1) + c];
+    if ((act >> (r * LPT)) & 1u) put<KIND>(out + (ia_w + r) * 210 + packed_index(X, X) + c, stage[r * (W | 1) + c]);
   }
   __syncwarp();
 }
@@ -698,20 +811,21 @@ template <int FORM, int KIND, typename R, int I>
 __device__ __forceinline__ void do_row_block(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
                                              const CR<R> &cM, uint64_t inv, bool active, int ia,
                                              typename StoreT<R>::T *stage, typename StoreT<R>::T *out) {
-  constexpr int W = 4 * (10 - I);
+  constexpr int W = 4 * (10 - I), LPT = lanes_per_tet(KIND);
   const int lane = threadIdx.x & 31;
   if (active)
-    compute_block_row<I, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane * (W | 1),
+    compute_block_row<I, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane / LPT * (W | 1),
                                         std::make_integer_sequence<int, 10 - I>{});
-  // the warp's 32 tets are consecutive assembled indices: lane r's is ia - lane + r
+  // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
   const unsigned act = __ballot_sync(0xffffffffu, active);
-  const int64_t ia_w = (int64_t)ia - lane;
+  const int64_t ia_w = (int64_t)ia - lane / LPT;
   __syncwarp();
 #pragma unroll 2
-  for (int it = 0; it < W; ++it) {
+  for (int it = 0; it < W / LPT; ++it) {
     const int e = it * 32 + lane;
     const int r = e / W, c = e - r * W;
-    if ((act >> r) & 1u) out[(ia_w + r) * kBlockValues + 4 * block_index(I, I) + c] = stage[r * (W | 1) + c];
+    if ((act >> (r * LPT)) & 1u)
+      put<KIND>(out + (ia_w + r) * kBlockValues + 4 * block_index(I, I) + c, stage[r * (W | 1) + c]);
   }
   __syncwarp();
 }
@@ -729,26 +843,34 @@ __device__ __forceinline__ void all_rows_block(const Tensors<KIND, R> &T, const 
 // LAYOUT 1: the packed canonical upper triangle [ia][210] (each unique
 //           entry computed once);
 // LAYOUT 2: the entity-pair blocks [ia][220] (the assembly path)
-// One CTA's 128 tets, assembled indices ia0 .. ia0 + 127 of the job a (every
-// thread of the CTA calls it with the same ia0).
-template <int FORM, int KIND, int LAYOUT>
-__device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsigned char *stage_raw) {
+// One CTA's tets (elem_tets_per_cta), from assembled index ia0 of the job a on
+// (every thread of the CTA calls it with the same ia0).
+// TK: the tensors' form. Returns whether any tet of the warp needs the
+// antisymmetric pass.
+template <int FORM, int KIND, int LAYOUT, int TK>
+__device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, unsigned char *stage_raw) {
   using R = typename FormReal<FORM>::T;
   using ST = typename StoreT<R>::T;
-  // values per lane: a row's stride is odd (in values), so the 32 lanes'
-  // stores of one value position fall in distinct shared-memory bank groups
+  constexpr int LPT = lanes_per_tet(TK);
+  // values per tet: a row's stride is odd (in values), so the lanes' stores of
+  // one value position fall in distinct shared-memory bank groups
   constexpr int STAGE = LAYOUT == 2 ? 41 : 21;
-  ST *stage = reinterpret_cast<ST *>(stage_raw) + (threadIdx.x >> 5) * (32 * STAGE);
+  ST *stage = reinterpret_cast<ST *>(stage_raw) + (threadIdx.x >> 5) * (32 / LPT * STAGE);
   ST *out = reinterpret_cast<ST *>(a.out);
-  const int64_t ia64 = ia0 + threadIdx.x;
+  const int64_t ia64 = ia0 + threadIdx.x / LPT;
   bool active = ia64 < a.nA;
   const int ia = (int)ia64;
   Geo G;
-  Tensors<KIND, R> T;
+  Tensors<TK, R> T;
   R mu[FORM == FORM_REF64 ? NMOM : 1];
+  if constexpr (FORM == FORM_REF64) {
+#pragma unroll
+    for (int i = 0; i < NMOM; ++i) mu[i] = (R)0;
+  }
   CR<R> cK{0, 0}, cM{0, 0};
   double sig = 1.0;
   uint64_t inv = 0;
+  bool asym = false;
   if (active) {
     int64_t it = a.tetids ? (int64_t)a.tetids[ia] : ia64;
     int64_t v[4];
@@ -773,7 +895,7 @@ __device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsi
       if constexpr (FORM != FORM_REF64) {
         good = exact_geometry(X, v, G);
       } else {
-        good = ref_geometry<R>(X, v, G, mu);
+        good = ref_geometry<LPT == 2, R>(X, v, G, mu);
       }
       if (!good) {
         flag(a.st, EMG_ST_DEGENERATE, ia64);
@@ -802,26 +924,55 @@ __device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsi
               mu3[3 * r + c] = (need && a.ur) ? ld_c64(a.ur, o) : C64{(r == c) ? 1.0 : 0.0, 0.0};
             }
           matinv3(mu3, minv);
-          cK = {(R)alpha.re, (R)alpha.im};
-          cM = {(R)beta.re, (R)beta.im};
-          build_cplx<KIND, R>(G, eps, minv, T);
+          if constexpr (LPT == 2) {
+            auto symmetric = [](const C64 t[9]) {
+              return t[1].re == t[3].re && t[1].im == t[3].im && t[2].re == t[6].re && t[2].im == t[6].im &&
+                     t[5].re == t[7].re && t[5].im == t[7].im;
+            };
+            asym = KIND == EMG_MAT_FULL && !(symmetric(eps) && symmetric(mu3));
+            double e[9], u[9];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) {
+              const C64 ce = cmul(beta, eps[i]), cu = cmul(alpha, minv[i]);
+              e[i] = (threadIdx.x & 1) ? ce.im : ce.re;
+              u[i] = (threadIdx.x & 1) ? cu.im : cu.re;
+            }
+            build_pair<TK, R>(G, e, u, T);
+          } else {
+            cK = {(R)alpha.re, (R)alpha.im};
+            cM = {(R)beta.re, (R)beta.im};
+            build_cplx<KIND, R>(G, eps, minv, T);
+          }
         }
       }
     }
   }
+  if constexpr (LPT == 2 && FORM == FORM_REF64) {  // both halves of the points
+#pragma unroll
+    for (int i = 0; i < NMOM; ++i) mu[i] += __shfl_xor_sync(0xffffffffu, mu[i], 1);
+  }
   if constexpr (LAYOUT == 0) {
-    all_rows<FORM, KIND, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out, std::make_integer_sequence<int, 20>{});
+    all_rows<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out, std::make_integer_sequence<int, 20>{});
   } else if constexpr (LAYOUT == 2) {
-    all_rows_block<FORM, KIND, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
+    all_rows_block<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
                                   std::make_integer_sequence<int, 10>{});
   } else {
-    all_rows_packed<FORM, KIND, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
+    all_rows_packed<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
                                    std::make_integer_sequence<int, 20>{});
   }
+  return TK == KIND_PAIR_FULL && __any_sync(0xffffffffu, asym);
+}
+
+template <int FORM, int KIND, int LAYOUT>
+__device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsigned char *stage_raw) {
+  constexpr int TK = tensor_kind(FORM, KIND);
+  const bool asym = element_pass<FORM, KIND, LAYOUT, TK>(a, ia0, stage_raw);
+  if constexpr (TK == KIND_PAIR_FULL)
+    if (asym) element_pass<FORM, KIND, LAYOUT, KIND_PAIR_ANTI>(a, ia0, stage_raw);
 }
 
 // CTAs per SM the compiler must fit. Measured on the 2.01M-tet box: the
-// FP64 forms at their natural 242-255 registers (two CTAs) beat every cap (a
+// isotropic FP64 forms at their natural 242-255 registers (two CTAs) beat every cap (a
 // three-CTA cap: 1.84 -> 3.68 ms, 1.9 KB of spills); the mixed form needs 88-254
 // registers with no cap (five CTAs per SM for the isotropic instance, set by
 // its 42 KB stage as much as by registers).
@@ -830,10 +981,16 @@ constexpr int elem_min_blocks() {
   return 1;
 }
 
+// tets of a CTA; elem_tets_per_cta for the host
+template <int FORM, int KIND>
+__host__ __device__ constexpr int elem_tets() {
+  return ELEM_THREADS / lanes_per_tet(tensor_kind(FORM, KIND));
+}
+
 template <int FORM, int KIND, int LAYOUT>
 __global__ void __launch_bounds__(ELEM_THREADS, elem_min_blocks<FORM, KIND>()) k_element(ElemArgs a) {
   extern __shared__ __align__(16) unsigned char stage_raw[];
-  element_cta<FORM, KIND, LAYOUT>(a, (int64_t)blockIdx.x * ELEM_THREADS, stage_raw);
+  element_cta<FORM, KIND, LAYOUT>(a, (int64_t)blockIdx.x * elem_tets<FORM, KIND>(), stage_raw);
 }
 
 // Several jobs (meshes, materials, coefficients, outputs) in one launch of
@@ -851,13 +1008,14 @@ __global__ void __launch_bounds__(ELEM_THREADS, elem_min_blocks<FORM, KIND>())
     else hi = mid - 1;
   }
   if (n_jobs <= 0 || b >= cta_start[n_jobs]) return;
-  element_cta<FORM, KIND, LAYOUT>(jobs[lo], (b - cta_start[lo]) * ELEM_THREADS, stage_raw);
+  element_cta<FORM, KIND, LAYOUT>(jobs[lo], (b - cta_start[lo]) * elem_tets<FORM, KIND>(), stage_raw);
 }
 
 template <int FORM, int KIND, int LAYOUT>
 int launch_element_t(const ElemArgs &a, cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
-  constexpr size_t smem = (size_t)ELEM_WARPS * 32 * (LAYOUT == 2 ? 41 : 21) * sizeof(ST);
+  constexpr size_t smem = (size_t)elem_tets<FORM, KIND>() * (LAYOUT == 2 ? 41 : 21) * sizeof(ST);
+  static_assert(elem_tets<FORM, KIND>() == elem_tets_per_cta(FORM, KIND), "the host's table of CTAs");
   // the attribute belongs to the current device: set once per device (benign
   // race: every thread that gets here sets the same value)
   static bool configured[64] = {false};
@@ -870,7 +1028,7 @@ int launch_element_t(const ElemArgs &a, cudaStream_t s) {
     if (dev < 64) configured[dev] = true;
   }
   if (a.nA == 0) return EMG_OK;
-  k_element<FORM, KIND, LAYOUT><<<grid_for(a.nA, ELEM_THREADS), ELEM_THREADS, smem, s>>>(a);
+  k_element<FORM, KIND, LAYOUT><<<grid_for(a.nA, elem_tets<FORM, KIND>()), ELEM_THREADS, smem, s>>>(a);
   return launch_check("k_element");
 }
 
@@ -878,7 +1036,7 @@ template <int FORM, int KIND, int LAYOUT>
 int launch_element_batch_t(const ElemArgs *d_jobs, const int64_t *d_cta_start, int n_jobs, int64_t total_ctas,
                            cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
-  constexpr size_t smem = (size_t)ELEM_WARPS * 32 * (LAYOUT == 2 ? 41 : 21) * sizeof(ST);  // element_cta's stage
+  constexpr size_t smem = (size_t)elem_tets<FORM, KIND>() * (LAYOUT == 2 ? 41 : 21) * sizeof(ST);  // element_cta's stage
   static bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
