@@ -619,19 +619,67 @@ __global__ void k_chunk_keys(const int32_t *ent_ptr, const Item *items, const do
   keys[c] = key;
 }
 
-// one compare-exchange step (k, j) of a bitonic sort of n2 = 2^m keys
-__global__ void k_bitonic_step(uint64_t *keys, int64_t n2, int64_t j, int64_t k) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n2) return;
-  const int64_t l = i ^ j;
-  if (l > i) {
-    const uint64_t a = keys[i], b = keys[l];
-    const bool up = (i & k) == 0;
-    if ((a > b) == up) {
-      keys[i] = b;
-      keys[l] = a;
+// Bitonic sort of n2 = 2^m keys. A CTA does every step within a tile of
+// SORT_TILE keys in shared memory: all stages up to the tile (k_sort_tiles), or
+// the steps j < SORT_TILE of stage k (k_sort_tail). The steps between tiles go
+// three to a launch, on the 8 keys a thread exchanges among themselves. 2^14 keys
+// (a port's forcing vector) take 3 launches instead of 105, 2^17 10 instead of 153.
+constexpr int SORT_TILE = 8192;
+constexpr int SORT_THREADS = 1024;
+
+__device__ __forceinline__ void sort_tile_steps(uint64_t *t, int tile, int64_t base, int64_t k, int j0) {
+  for (int j = j0; j > 0; j >>= 1) {
+    __syncthreads();
+    for (int c = threadIdx.x; c < tile / 2; c += SORT_THREADS) {
+      const int i = ((c & ~(j - 1)) << 1) | (c & (j - 1)), l = i | j;
+      const uint64_t a = t[i], b = t[l];
+      if ((a > b) == (((base + i) & k) == 0)) {
+        t[i] = b;
+        t[l] = a;
+      }
     }
   }
+}
+
+// ALL: sort the tile (all n2 keys, if fewer) from scratch; else stage k's last steps
+template <bool ALL>
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_tile(uint64_t *keys, int64_t n2, int64_t k) {
+  extern __shared__ uint64_t sort_keys[];
+  const int tile = (int)min((int64_t)SORT_TILE, n2);
+  const int64_t base = (int64_t)blockIdx.x * tile;
+  for (int i = threadIdx.x; i < tile; i += SORT_THREADS) sort_keys[i] = keys[base + i];
+  if (ALL) {
+    for (int s = 2; s <= tile; s <<= 1) sort_tile_steps(sort_keys, tile, base, s, s >> 1);
+  } else {
+    sort_tile_steps(sort_keys, tile, base, k, tile >> 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < tile; i += SORT_THREADS) keys[base + i] = sort_keys[i];
+}
+
+// steps j, j/2, ..., j/2^(STEPS-1) of stage k: a thread's 2^STEPS keys lie j/2^(STEPS-1) apart
+template <int STEPS>
+__global__ void __launch_bounds__(256) k_sort_steps(uint64_t *keys, int64_t n2, int64_t j, int64_t k) {
+  constexpr int M = 1 << STEPS;
+  const int64_t lo = j >> (STEPS - 1);  // the smallest of the steps
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n2 / M) return;
+  const int64_t i0 = (c / lo) * (lo * M) + c % lo;
+  uint64_t v[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) v[m] = keys[i0 + m * lo];
+  const bool up = (i0 & k) == 0;  // k > j: the same for all of them
+#pragma unroll
+  for (int h = M / 2; h > 0; h >>= 1)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      if (!(m & h) && (v[m] > v[m | h]) == up) {
+        const uint64_t t = v[m];
+        v[m] = v[m | h];
+        v[m | h] = t;
+      }
+#pragma unroll
+  for (int m = 0; m < M; ++m) keys[i0 + m * lo] = v[m];
 }
 
 // the new order; block layout: the chunk descriptors (by_chunk: in chunk
@@ -809,13 +857,36 @@ int plan_finish(const emg_plan *p, const int32_t *d_t2e, const int32_t *d_t2t, c
 
 int sort_u64(uint64_t *keys, int64_t n2, cudaStream_t s) {
   if (n2 & (n2 - 1)) return fail(EMG_EINVAL, "sort length %lld is not a power of two", (long long)n2);
-  for (int64_t k = 2; k <= n2; k <<= 1)
-    for (int64_t j = k >> 1; j > 0; j >>= 1) {
-      k_bitonic_step<<<grid_for(n2, 256), 256, 0, s>>>(keys, n2, j, k);
-      const int rc = launch_check("k_bitonic_step");
-      if (rc) return rc;
+  if (n2 < 2) return EMG_OK;
+  constexpr int smem = SORT_TILE * 8;
+  // the attribute belongs to the current device: set once per device (benign
+  // race: every thread that gets here sets the same value)
+  static bool configured[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
+  if (dev >= 64 || !configured[dev]) {
+    CUDA_TRY(cudaFuncSetAttribute(k_sort_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CUDA_TRY(cudaFuncSetAttribute(k_sort_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (dev < 64) configured[dev] = true;
+  }
+  const int tiles = grid_for(n2, SORT_TILE);
+  k_sort_tile<true><<<tiles, SORT_THREADS, smem, s>>>(keys, n2, 0);
+  int rc = launch_check("k_sort_tile");
+  for (int64_t k = 2 * SORT_TILE; k <= n2 && !rc; k <<= 1) {
+    for (int64_t j = k >> 1; j >= SORT_TILE && !rc;) {
+      const int steps = j >= 4 * SORT_TILE ? 3 : (j >= 2 * SORT_TILE ? 2 : 1);
+      const int g = grid_for(n2 >> steps, 256);
+      if (steps == 3) k_sort_steps<3><<<g, 256, 0, s>>>(keys, n2, j, k);
+      else if (steps == 2) k_sort_steps<2><<<g, 256, 0, s>>>(keys, n2, j, k);
+      else k_sort_steps<1><<<g, 256, 0, s>>>(keys, n2, j, k);
+      rc = launch_check("k_sort_steps");
+      j >>= steps;
     }
-  return EMG_OK;
+    if (rc) return rc;
+    k_sort_tile<false><<<tiles, SORT_THREADS, smem, s>>>(keys, n2, k);
+    rc = launch_check("k_sort_tile");
+  }
+  return rc;
 }
 
 int plan_order(const emg_plan *p, void *d_plan, const double *nodes, int64_t nN, const int32_t *tets,
