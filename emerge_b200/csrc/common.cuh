@@ -124,6 +124,31 @@ __device__ __forceinline__ void flag(int64_t *st, int64_t bit, int64_t index) {
   }
 }
 
+// ascending sort of a warp's 32 K keys (bitonic network), key i in register i / 32 of lane i % 32
+template <int K>
+__device__ __forceinline__ void warp_sort(uint64_t (&k)[K]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int size = 2; size <= 32 * K; size <<= 1)
+#pragma unroll
+    for (int j = size >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < K; ++r) {
+        const bool up = ((r * 32 + lane) & size) == 0;
+        if (j >= 32) {
+          const int o = r | (j >> 5);
+          if (o != r && (k[r] > k[o]) == up) {
+            const uint64_t t = k[r];
+            k[r] = k[o];
+            k[o] = t;
+          }
+        } else {
+          const uint64_t o = __shfl_xor_sync(0xffffffffu, k[r], j);
+          k[r] = (((lane & j) == 0) == up) == (k[r] < o) ? k[r] : o;
+        }
+      }
+}
+
 // Item record, 16 bytes: assembled tet index, entity slot (0-5 edge, 6-9 face)
 // of the owning entity in that tet, and for each of the tet's 10 entity slots
 // its index in the owner's sorted adjacent-edge (slots 0-5) or adjacent-face

@@ -44,31 +44,6 @@ __device__ __forceinline__ uint64_t coo_key(const int32_t *rows, int32_t slot) {
   return ((uint64_t)(uint32_t)rows[slot] << 32) | (uint32_t)slot;
 }
 
-// ascending sort of the keys, key i in register i / 32 of lane i % 32
-template <int K>
-__device__ __forceinline__ void warp_sort(uint64_t (&k)[K]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int size = 2; size <= 32 * K; size <<= 1)
-#pragma unroll
-    for (int j = size >> 1; j > 0; j >>= 1)
-#pragma unroll
-      for (int r = 0; r < K; ++r) {
-        const bool up = ((r * 32 + lane) & size) == 0;
-        if (j >= 32) {
-          const int o = r | (j >> 5);
-          if (o != r && (k[r] > k[o]) == up) {
-            const uint64_t t = k[r];
-            k[r] = k[o];
-            k[o] = t;
-          }
-        } else {
-          const uint64_t o = __shfl_xor_sync(0xffffffffu, k[r], j);
-          k[r] = (((lane & j) == 0) == up) == (k[r] < o) ? k[r] : o;
-        }
-      }
-}
-
 // sorts the column's n <= 32 K slots perm[0..n); returns its distinct rows
 template <int K>
 __device__ __forceinline__ int32_t sort_column(const int32_t *rows, int64_t N, int32_t *perm, int n, int64_t *st) {

@@ -192,107 +192,160 @@ __global__ void k_sort_items(const int32_t *ent_ptr, int64_t n_ent, Item *items)
   }
 }
 
-// Warp per entity. Candidates = the 6 edges / 4 faces of every incident tet;
-// unique values counted (count pass) or ranked (fill pass) by comparison in
-// shared memory.
+// Warp per entity. Candidates = the 6 edges and 4 faces of every incident tet,
+// faces marked to come after all edges: sorted with their place (in registers; in
+// shared memory past 120), so that a candidate's rank among the distinct values,
+// its position in the item, is the number of first ones up to it. k_entity_rows
+// does this for the column lengths and the positions; k_entity_indices then
+// writes the rows. Comparing all candidates with each other, once to count and
+// once to rank, took 152 + 313 us at 103,680 tets; this 154 + 106. Bound: latency
+// (item -> tet -> candidate).
 constexpr int ROWS_WARPS = 4;
-constexpr int CAND_CAP = 640;   // edge candidates per entity (6 per tet) => up to 106 incident tets
-constexpr int CAND_CAP_F = 432; // face candidates (4 per tet)
+constexpr int MAX_ITEMS = 106;  // incident tets of an entity
+constexpr int BIG_ITEMS = 12;   // up to here its candidates are sorted in registers
 
-template <bool FILL>
-__global__ void __launch_bounds__(ROWS_WARPS * 32)
-    k_entity_rows(const int32_t *t2e, const int32_t *t2t, const int32_t *tetids, int64_t nT, int64_t E, int64_t F,
-                  const int32_t *ent_ptr, Item *items, int64_t n_ent, int32_t *col_len, uint32_t *ent_cnt,
-                  const int32_t *indptr, int32_t *indices, int64_t *st) {
-  __shared__ int32_t cand_e[ROWS_WARPS][CAND_CAP];
-  __shared__ int32_t cand_f[ROWS_WARPS][CAND_CAP_F];
-  __shared__ uint8_t first_e[ROWS_WARPS][CAND_CAP];
-  __shared__ uint8_t first_f[ROWS_WARPS][CAND_CAP_F];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int64_t x = (int64_t)blockIdx.x * ROWS_WARPS + w;
-  if (x >= n_ent) return;
-  int32_t b = ent_ptr[x], e = ent_ptr[x + 1];
-  int nitem = e - b;
-  int ne = nitem * 6, nf = nitem * 4;
-  if (ne > CAND_CAP || nf > CAND_CAP_F) {
-    if (lane == 0) flag(st, EMG_ST_CAPACITY, x);
-    return;
+// ranks sorted candidates, 32 a round (key = face << 63 | value << 32 | place), into
+// the items; counts the distinct edges and faces
+struct CandRank {
+  int ue, uf;
+  uint32_t last;
+  __device__ __forceinline__ void round(uint64_t key, bool in, bool start, Item *items) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t v = (uint32_t)(key >> 32), place = (uint32_t)key;
+    uint32_t before = __shfl_up_sync(0xffffffffu, v, 1);
+    if (lane == 0) before = last;
+    const bool first = in && ((start && lane == 0) || v != before), face = v >> 31;
+    const unsigned me = __ballot_sync(0xffffffffu, first && !face), mf = __ballot_sync(0xffffffffu, first && face);
+    const unsigned upto = 0xffffffffu >> (31 - lane);
+    // a rank over MAX_ADJ does not fit: the caller flags it
+    if (in) items[place / 10].pos[place % 10] = (uint8_t)((face ? uf + __popc(mf & upto) : ue + __popc(me & upto)) - 1);
+    ue += __popc(me);
+    uf += __popc(mf);
+    last = __shfl_sync(0xffffffffu, v, 31);
   }
-  int32_t *ce = cand_e[w], *cf = cand_f[w];
-  uint8_t *fe = first_e[w], *ff = first_f[w];
-  for (int i = lane; i < ne; i += 32) {
-    int64_t it = tet_of(tetids, items[b + i / 6].ia);
-    ce[i] = t2e[(int64_t)(i % 6) * nT + it];
-  }
-  for (int i = lane; i < nf; i += 32) {
-    int64_t it = tet_of(tetids, items[b + i / 4].ia);
-    cf[i] = t2t[(int64_t)(i % 4) * nT + it];
-  }
-  __syncwarp();
-  // first occurrences -> number of distinct adjacent edges / faces
-  int ue = 0, uf = 0;
-  for (int i = lane; i < ne; i += 32) {
-    int32_t v = ce[i];
-    bool first = true;
-    for (int j = 0; j < i; ++j) first &= (ce[j] != v);
-    fe[i] = first;
-    ue += first;
-  }
-  for (int i = lane; i < nf; i += 32) {
-    int32_t v = cf[i];
-    bool first = true;
-    for (int j = 0; j < i; ++j) first &= (cf[j] != v);
-    ff[i] = first;
-    uf += first;
-  }
+};
+
+template <int K, typename Load>
+__device__ __forceinline__ void rank_candidates(int n, Item *items, CandRank &c, Load load) {
+  const int lane = threadIdx.x & 31;
+  uint64_t k[K];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ue += __shfl_xor_sync(0xffffffffu, ue, o);
-    uf += __shfl_xor_sync(0xffffffffu, uf, o);
-  }
-  if (ue > MAX_ADJ || uf > MAX_ADJ) {
-    if (lane == 0) flag(st, EMG_ST_CAPACITY, x);
+  for (int r = 0; r < K; ++r) k[r] = r * 32 + lane < n ? load(r * 32 + lane) : ~0ull;
+  warp_sort<K>(k);
+#pragma unroll
+  for (int r = 0; r < K; ++r) c.round(k[r], r * 32 + lane < n, r == 0, items);
+}
+
+// one entity, up to 10 BIG_ITEMS candidates in registers or, `buf`, any number
+struct RowsArgs {
+  const int32_t *t2e, *t2t, *tetids;
+  int64_t nT, E, F;
+  const int32_t *ent_ptr;
+  Item *items;
+  int64_t n_ent;
+  int32_t *col_len;
+  uint32_t *ent_cnt;
+  int64_t *st;
+};
+
+template <bool BIG>
+__device__ __forceinline__ void entity_rows(const RowsArgs &a, int64_t x, uint64_t *buf) {
+  const int lane = threadIdx.x & 31;
+  const int32_t b = a.ent_ptr[x];
+  const int nitem = a.ent_ptr[x + 1] - b, n = 10 * nitem;
+  if (!BIG && nitem > BIG_ITEMS) return;  // k_big_entity_rows
+  if (BIG && nitem > MAX_ITEMS) {
+    if (lane == 0) flag(a.st, EMG_ST_CAPACITY, x);
     return;
   }
+  Item *own = a.items + b;
+  auto load = [&](int i) {
+    const int s = i % 10;
+    const int64_t it = tet_of(a.tetids, own[i / 10].ia);
+    const uint32_t v =
+        s < 6 ? (uint32_t)a.t2e[(int64_t)s * a.nT + it] : 0x80000000u | (uint32_t)a.t2t[(int64_t)(s - 6) * a.nT + it];
+    return ((uint64_t)v << 32) | (uint32_t)i;
+  };
+  CandRank c{0, 0, 0};
+  if constexpr (!BIG) {
+    if (n <= 32) rank_candidates<1>(n, own, c, load);
+    else if (n <= 64) rank_candidates<2>(n, own, c, load);
+    else rank_candidates<4>(n, own, c, load);
+  } else {
+    for (int i = lane; i < n; i += 32) buf[i] = load(i);
+    __syncwarp();
+    // comparators that all put the smaller key first: those past the end are left out
+    for (int size = 2; (size >> 1) < n; size <<= 1)
+      for (int j = size >> 1; j > 0; j >>= 1) {
+        for (int k = lane; k < (n + 2 * j - 1) / (2 * j) * j; k += 32) {
+          const int block = k / j * (2 * j), at = k % j;
+          const int i = block + at, o = j == (size >> 1) ? block + 2 * j - 1 - at : i + j;
+          if (o < n && buf[i] > buf[o]) {
+            const uint64_t t = buf[i];
+            buf[i] = buf[o];
+            buf[o] = t;
+          }
+        }
+        __syncwarp();
+      }
+    for (int i0 = 0; i0 < n; i0 += 32) c.round(i0 + lane < n ? buf[i0 + lane] : ~0ull, i0 + lane < n, i0 == 0, own);
+    __syncwarp();
+  }
+  if (lane != 0) return;
+  if (c.ue > MAX_ADJ || c.uf > MAX_ADJ) {
+    flag(a.st, EMG_ST_CAPACITY, x);
+    return;
+  }
+  const bool is_edge = x < a.E;
+  const int32_t L = 2 * (c.ue + c.uf);
+  a.col_len[is_edge ? x : a.E + x] = L;              // 2E + (x - E)
+  a.col_len[is_edge ? x + a.E : a.E + a.F + x] = L;  // 2E + F + (x - E)
+  a.ent_cnt[x] = (uint32_t)c.ue | ((uint32_t)c.uf << 16);
+}
+
+__global__ void __launch_bounds__(ROWS_WARPS * 32) k_entity_rows(const RowsArgs a) {
+  const int64_t x = (int64_t)blockIdx.x * ROWS_WARPS + (threadIdx.x >> 5);
+  if (x < a.n_ent) entity_rows<false>(a, x, nullptr);
+}
+
+// the entities with more than BIG_ITEMS incident tets, few in any mesh: a warp
+// looks through 32 entities at a time
+__global__ void __launch_bounds__(ROWS_WARPS * 32) k_big_entity_rows(const RowsArgs a) {
+  __shared__ uint64_t bufs[ROWS_WARPS][10 * MAX_ITEMS];
+  const int lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * ROWS_WARPS * 32;
+  for (int64_t x0 = ((int64_t)blockIdx.x * ROWS_WARPS + (threadIdx.x >> 5)) * 32; x0 < a.n_ent; x0 += step) {
+    const int64_t x = x0 + lane;
+    unsigned big = __ballot_sync(0xffffffffu, x < a.n_ent && a.ent_ptr[x + 1] - a.ent_ptr[x] > BIG_ITEMS);
+    for (; big; big &= big - 1) entity_rows<true>(a, x0 + __ffs(big) - 1, bufs[threadIdx.x >> 5]);
+  }
+}
+
+// the rows of the four column blocks: every candidate writes its value at its rank
+__global__ void __launch_bounds__(ROWS_WARPS * 32)
+    k_entity_indices(const int32_t *t2e, const int32_t *t2t, const int32_t *tetids, int64_t nT, int64_t E, int64_t F,
+                     const int32_t *ent_ptr, const Item *items, int64_t n_ent, const uint32_t *ent_cnt,
+                     const int32_t *indptr, int32_t *indices) {
+  const int lane = threadIdx.x & 31;
+  const int64_t x = (int64_t)blockIdx.x * ROWS_WARPS + (threadIdx.x >> 5);
+  if (x >= n_ent) return;
+  const int32_t b = ent_ptr[x];
+  const int n = 10 * (ent_ptr[x + 1] - b);
+  const uint32_t c = ent_cnt[x];
+  const int ue = (int)(c & 0xffffu), uf = (int)(c >> 16);
   const bool is_edge = x < E;
-  const int64_t c0 = is_edge ? x : E + x;          // 2E + (x - E)
-  const int64_t c1 = is_edge ? x + E : E + F + x;  // 2E + F + (x - E)
-  if (!FILL) {
-    if (lane == 0) {
-      int32_t L = 2 * (ue + uf);
-      col_len[c0] = L;
-      col_len[c1] = L;
-      ent_cnt[x] = (uint32_t)ue | ((uint32_t)uf << 16);
-    }
-    return;
-  }
-  __syncwarp();
-  // rank = number of distinct smaller values; rows of the four column blocks
-  const int64_t s0 = indptr[c0], s1 = indptr[c1];
-  for (int i = lane; i < ne; i += 32) {
-    int32_t v = ce[i];
-    int r = 0;
-    for (int j = 0; j < ne; ++j) r += (fe[j] && ce[j] < v) ? 1 : 0;
-    if (fe[i]) {
-      indices[s0 + r] = v;
-      indices[s0 + ue + r] = v + (int32_t)E;
-      indices[s1 + r] = v;
-      indices[s1 + ue + r] = v + (int32_t)E;
-    }
-    items[b + i / 6].pos[i % 6] = (uint8_t)r;
-  }
-  for (int i = lane; i < nf; i += 32) {
-    int32_t v = cf[i];
-    int r = 0;
-    for (int j = 0; j < nf; ++j) r += (ff[j] && cf[j] < v) ? 1 : 0;
-    if (ff[i]) {
-      int32_t r0 = v + 2 * (int32_t)E, r1 = v + 2 * (int32_t)E + (int32_t)F;
-      indices[s0 + 2 * ue + r] = r0;
-      indices[s0 + 2 * ue + uf + r] = r1;
-      indices[s1 + 2 * ue + r] = r0;
-      indices[s1 + 2 * ue + uf + r] = r1;
-    }
-    items[b + i / 4].pos[6 + i % 4] = (uint8_t)r;
+  const int64_t s0 = indptr[is_edge ? x : E + x], s1 = indptr[is_edge ? x + E : E + F + x];
+  for (int i = lane; i < n; i += 32) {
+    const int k = i / 10, s = i % 10;
+    const Item &rec = items[b + k];
+    const int64_t it = tet_of(tetids, rec.ia);
+    const int r = rec.pos[s];
+    const bool e = s < 6;
+    const int32_t v = e ? t2e[(int64_t)s * nT + it] : t2t[(int64_t)(s - 6) * nT + it];
+    const int at = e ? r : 2 * ue + r, part = e ? ue : uf;
+    const int32_t r0 = e ? v : v + 2 * (int32_t)E, r1 = e ? v + (int32_t)E : v + 2 * (int32_t)E + (int32_t)F;
+    indices[s0 + at] = indices[s1 + at] = r0;
+    indices[s0 + at + part] = indices[s1 + at + part] = r1;
   }
 }
 
@@ -402,7 +455,15 @@ __global__ void __launch_bounds__(CC_WARPS * 32)
 // items of the chunk entity that hold the same row entity (the same position
 // byte) give the length of the row pair's list and the block's place in it, in
 // item order, so each output sums its contributions in the order of the packed
-// lists. Layout of the records: common.cuh.
+// lists. Layout of the records: common.cuh. A tet's canonical entities come from
+// a table of its vertex ranks that each CTA lays out once for all its chunks.
+// 103,680 tets: 192 us (683 with them worked out per lane, 351 for a serial walk
+// over the items).
+__device__ __forceinline__ uint32_t item_byte(const uint4 &o, int i) {  // byte i of an item
+  const uint32_t w = i < 8 ? (i < 4 ? o.x : o.y) : (i < 12 ? o.z : o.w);
+  return (w >> (8 * (i & 3))) & 0xffu;
+}
+
 __global__ void __launch_bounds__(CC_WARPS * 32)
     k_chunk_blocks(const int32_t *ent_ptr, const Item *items, const uint32_t *ent_cnt, int64_t E, int64_t F,
                    const int32_t *indptr, uint32_t *brec, int64_t *st) {
@@ -410,78 +471,93 @@ __global__ void __launch_bounds__(CC_WARPS * 32)
     int32_t ptr[CHUNK + 1], c0[CHUNK + 1], ne[CHUNK], n_long;
   };
   __shared__ Meta meta[CC_WARPS];
+  __shared__ uint8_t canon[256][12];  // canonical entity of slot s (0..9) by the tet's ranks byte
+  for (int i = threadIdx.x; i < 2560; i += CC_WARPS * 32) {
+    const int ranks = i / 10, s = i % 10;
+    canon[ranks][s] = (uint8_t)(s < 6 ? canon_dof(ranks, s) : canon_dof(ranks, 12 + (s - 6)) - 6);
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   Meta &m = meta[threadIdx.x >> 5];
-  const int64_t chunk = (int64_t)blockIdx.x * CC_WARPS + (threadIdx.x >> 5);
-  const int64_t nec = n_edge_chunks(E);
-  if (chunk >= n_chunks(E, F)) return;
-  const bool edges = chunk < nec;
-  const int64_t x0 = edges ? chunk * CHUNK : E + (chunk - nec) * CHUNK;
-  const int nx = (int)min((int64_t)CHUNK, (edges ? E : E + F) - x0);
-  const int64_t cb0 = edges ? x0 : E + x0;
-  if (lane <= nx) {
-    m.ptr[lane] = ent_ptr[x0 + lane];
-    m.c0[lane] = indptr[cb0 + lane];
-  }
-  if (lane < nx) m.ne[lane] = (int32_t)(ent_cnt[x0 + lane] & 0xffffu);
-  if (lane == 0) m.n_long = 0;
-  __syncwarp();
-  const int32_t I0 = m.ptr[0], nI = m.ptr[nx] - I0, A0 = m.c0[0];
-  const int Lsum = m.c0[nx] - A0, H = Lsum / 2;
-  if (Lsum > CHUNK_MAX_POS || nI > CHUNK_MAX_ITEMS) {
-    if (lane == 0) flag(st, EMG_ST_CAPACITY, x0);
-    return;
-  }
-  uint32_t *words = brec + (int64_t)kPairWords * I0;
-  uint2 *pairs = reinterpret_cast<uint2 *>(words);
+  const int64_t nec = n_edge_chunks(E), nch = n_chunks(E, F);
   const uint4 *raw = reinterpret_cast<const uint4 *>(items);
-  auto word_of = [&](const Item &rec, int r) {
-    const int s = rec.slot;
-    const int cb = s < 6 ? canon_dof(rec.ranks, s) : canon_dof(rec.ranks, 12 + (s - 6)) - 6;
-    const int ca = r < 6 ? canon_dof(rec.ranks, r) : canon_dof(rec.ranks, 12 + (r - 6)) - 6;
-    const int lo = ca < cb ? ca : cb, hi = ca < cb ? cb : ca;
-    return (uint32_t)((int64_t)rec.ia * 55 + block_index(lo, hi)) | (ca > cb ? 0x80000000u : 0u);
+  // block number of item o for row slot r, bit 31 when it is stored transposed
+  auto word_of = [&](const uint4 &o, int r) {
+    const uint8_t *of = canon[item_byte(o, 15)];
+    const int ca = of[r], cb = of[item_byte(o, 4)];
+    const int lo = min(ca, cb), hi = max(ca, cb);
+    return (o.x * 55u + (uint32_t)block_index(lo, hi)) | (ca > cb ? 0x80000000u : 0u);
   };
-  for (int t = lane; t < 10 * nI; t += 32) {
-    const int k = I0 + t / 10, r = t % 10;
-    int e = 0;
-    for (int q = 1; q < nx; ++q) e = k >= m.ptr[q] ? q : e;
-    const Item rec = items[k];
-    const uint32_t same = rec.pos[r] * 0x01010101u;
-    // bytes of an item: slot at 4, pos[0..9] at 5..14 (edges, then faces)
-    auto holds = [&](const uint4 &o) {
-      return r < 6 ? (__vcmpeq4(o.y, same) & 0xffffff00u) | (__vcmpeq4(o.z, same) & 0x00ffffffu)
-                   : (__vcmpeq4(o.z, same) & 0xff000000u) | (__vcmpeq4(o.w, same) & 0x00ffffffu);
-    };
-    const uint32_t word = word_of(rec, r);
-    int total = 0, rank = 0;
-    bool mixed = false;  // stored different ways round: only with inconsistent topology arrays
-    for (int i = m.ptr[e]; i < m.ptr[e + 1]; ++i)
-      if (holds(raw[i])) {
-        ++total;
-        rank += i < k ? 1 : 0;
-        if (i != k)
-          for (int p = r < 6 ? 0 : 6; p < (r < 6 ? 6 : 10); ++p)
-            if (items[i].pos[p] == rec.pos[r]) mixed = mixed || ((word_of(items[i], p) ^ word) >> 31);
-      }
-    const int h = (m.c0[e] - A0) / 2 + (r < 6 ? 0 : m.ne[e]) + rec.pos[r];
-    const bool self = r == rec.slot;  // the entity's pair with itself: every item has one
-    if (self) words[2 * H + (k - I0)] = word;
-    if (total <= 2 && !mixed) {
-      if (total == 1) pairs[h] = make_uint2(word, kBlockNone);
-      else words[2 * h + rank] = word;
-    } else if (rank == 0) {  // one lane writes the whole list
-      int off = 0;
-      if (!self) {
-        off = 2 * H + nI + atomicAdd(&m.n_long, total);
-        uint32_t *list = words + off;
-        for (int i = m.ptr[e]; i < m.ptr[e + 1]; ++i) {
-          const Item o = items[i];
-          for (int p = r < 6 ? 0 : 6; p < (r < 6 ? 6 : 10); ++p)
-            if (o.pos[p] == rec.pos[r]) *list++ = word_of(o, p);
+  for (int64_t chunk = (int64_t)blockIdx.x * CC_WARPS + (threadIdx.x >> 5); chunk < nch;
+       chunk += (int64_t)gridDim.x * CC_WARPS) {
+    const bool edges = chunk < nec;
+    const int64_t x0 = edges ? chunk * CHUNK : E + (chunk - nec) * CHUNK;
+    const int nx = (int)min((int64_t)CHUNK, (edges ? E : E + F) - x0);
+    const int64_t cb0 = edges ? x0 : E + x0;
+    __syncwarp();
+    if (lane <= CHUNK) {  // past the chunk's last entity: its end
+      m.ptr[lane] = ent_ptr[x0 + min(lane, nx)];
+      m.c0[lane] = indptr[cb0 + min(lane, nx)];
+    }
+    if (lane < nx) m.ne[lane] = (int32_t)(ent_cnt[x0 + lane] & 0xffffu);
+    if (lane == 0) m.n_long = 0;
+    __syncwarp();
+    const int32_t I0 = m.ptr[0], nI = m.ptr[CHUNK] - I0, A0 = m.c0[0];
+    const int Lsum = m.c0[CHUNK] - A0, H = Lsum / 2;
+    if (Lsum > CHUNK_MAX_POS || nI > CHUNK_MAX_ITEMS) {
+      if (lane == 0) flag(st, EMG_ST_CAPACITY, x0);
+      continue;
+    }
+    uint32_t *words = brec + (int64_t)kPairWords * I0;
+    uint2 *pairs = reinterpret_cast<uint2 *>(words);
+    for (int t = lane; t < 10 * nI; t += 32) {
+      const int k = I0 + t / 10, r = t % 10;
+      int e = k >= m.ptr[4] ? 4 : 0;
+      e += k >= m.ptr[e + 2] ? 2 : 0;
+      e += k >= m.ptr[e + 1] ? 1 : 0;
+      const uint4 own = raw[k];
+      const uint32_t pos = item_byte(own, 5 + r), same = pos * 0x01010101u;
+      // bytes of an item: slot at 4, pos[0..9] at 5..14 (edges, then faces), ranks at 15
+      const uint32_t my = r < 6 ? 0xffffff00u : 0u, mz = r < 6 ? 0x00ffffffu : 0xff000000u, mw = r < 6 ? 0u : 0x00ffffffu;
+      const int i0 = m.ptr[e], i1 = m.ptr[e + 1];
+      int total = 0, rank = 0, other = k, other_r = r;
+      for (int i = i0; i < i1; ++i) {
+        const uint4 o = raw[i];
+        const uint32_t hy = __vcmpeq4(o.y, same) & my, hz = __vcmpeq4(o.z, same) & mz, hw = __vcmpeq4(o.w, same) & mw;
+        if (hy | hz | hw) {
+          ++total;
+          rank += i < k ? 1 : 0;
+          if (i != k) {
+            other = i;  // its row slot: the first matching byte, less the five before pos
+            other_r = (hy ? __ffs(hy) / 8 : (hz ? 4 + __ffs(hz) / 8 : 8 + __ffs(hw) / 8)) - 1;
+          }
         }
       }
-      pairs[h] = make_uint2(self ? 0u : (uint32_t)off | ((uint32_t)total << 16), kBlockLong);
+      const int h = (m.c0[e] - A0) / 2 + (r < 6 ? 0 : m.ne[e]) + (int)pos;
+      const uint32_t word = word_of(own, r);
+      const bool self = r == (int)item_byte(own, 4);  // the entity's pair with itself: every item has one
+      if (self) words[2 * H + (k - I0)] = word;
+      // two blocks stored different ways round: only with inconsistent topology arrays
+      const bool differ = total == 2 && ((word_of(raw[other], other_r) ^ word) >> 31);
+      if (total <= 2 && !differ) {
+        if (total == 1) pairs[h] = make_uint2(word, kBlockNone);
+        else words[2 * h + rank] = word;
+      } else if (rank == 0) {  // one lane writes the whole list
+        int off = 0;
+        if (!self) {
+          off = 2 * H + nI + atomicAdd(&m.n_long, total);
+          uint32_t *list = words + off;
+          for (int i = i0; i < i1; ++i) {
+            const uint4 o = raw[i];
+            for (int p = r < 6 ? 0 : 6; p < (r < 6 ? 6 : 10); ++p)
+              if (item_byte(o, 5 + p) == pos) {
+                *list++ = word_of(o, p);
+                break;
+              }
+          }
+        }
+        pairs[h] = make_uint2(self ? 0u : (uint32_t)off | ((uint32_t)total << 16), kBlockLong);
+      }
     }
   }
 }
@@ -561,15 +637,17 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const double *nodes, int64
   if (threadIdx.x < 6) part[blockIdx.x * 6 + threadIdx.x] = sm[threadIdx.x][0];
 }
 
+// a warp per bound
 __global__ void k_bbox_final(const double *part, int nblk, double *box) {
-  if (threadIdx.x < 6) {
-    double v = part[threadIdx.x];
-    for (int b = 1; b < nblk; ++b) {
-      const double x = part[b * 6 + threadIdx.x];
-      v = threadIdx.x < 3 ? fmin(v, x) : fmax(v, x);
-    }
-    box[threadIdx.x] = v;
+  const int d = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = d < 3 ? INFINITY : -INFINITY;
+  for (int b = lane; b < nblk; b += 32) v = d < 3 ? fmin(v, part[b * 6 + d]) : fmax(v, part[b * 6 + d]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double x = __shfl_xor_sync(0xffffffffu, v, o);
+    v = d < 3 ? fmin(v, x) : fmax(v, x);
   }
+  if (lane == 0) box[d] = v;
 }
 
 __device__ __forceinline__ uint32_t spread_bits10(uint32_t x) {  // bit i -> bit 3i
@@ -623,9 +701,11 @@ __global__ void k_chunk_keys(const int32_t *ent_ptr, const Item *items, const do
 // SORT_TILE keys in shared memory: all stages up to the tile (k_sort_tiles), or
 // the steps j < SORT_TILE of stage k (k_sort_tail). The steps between tiles go
 // three to a launch, on the 8 keys a thread exchanges among themselves. 2^14 keys
-// (a port's forcing vector) take 3 launches instead of 105, 2^17 10 instead of 153.
-constexpr int SORT_TILE = 8192;
-constexpr int SORT_THREADS = 1024;
+// (a port's forcing vector) take 7 launches and 40 us instead of 105 and 176, 2^16
+// and 2^17 30 and 160 us instead of 289 and 510. Tiles of 8,192 keys and 1,024
+// threads: fewer launches, but 87 and 293 us on the few SMs that have a tile.
+constexpr int SORT_TILE = 2048;
+constexpr int SORT_THREADS = 512;
 
 __device__ __forceinline__ void sort_tile_steps(uint64_t *t, int tile, int64_t base, int64_t k, int j0) {
   for (int j = j0; j > 0; j >>= 1) {
@@ -800,10 +880,13 @@ int plan_build(emg_plan *p, const int32_t *d_tets, const int32_t *d_t2e, const i
   if (p->n_ent > 0) {
     k_sort_items<<<grid_for(p->n_ent, 256), 256, 0, s>>>(ent_ptr, p->n_ent, items);
     if ((rc = launch_check("k_sort_items"))) return rc;
-    k_entity_rows<false><<<grid_for(p->n_ent, ROWS_WARPS), ROWS_WARPS * 32, 0, s>>>(
-        d_t2e, d_t2t, d_tetids, p->n_tets, p->n_edges, p->n_tris, ent_ptr, items, p->n_ent, col_len, ent_cnt,
-        nullptr, nullptr, d_status);
-    if ((rc = launch_check("k_entity_rows<count>"))) return rc;
+    const RowsArgs ra{d_t2e, d_t2t, d_tetids, p->n_tets, p->n_edges, p->n_tris, ent_ptr, items, p->n_ent, col_len,
+                      ent_cnt, d_status};
+    k_entity_rows<<<grid_for(p->n_ent, ROWS_WARPS), ROWS_WARPS * 32, 0, s>>>(ra);
+    if ((rc = launch_check("k_entity_rows"))) return rc;
+    const int g = grid_for(p->n_ent, ROWS_WARPS * 32);
+    k_big_entity_rows<<<g < persistent_ctas(4) ? g : persistent_ctas(4), ROWS_WARPS * 32, 0, s>>>(ra);
+    if ((rc = launch_check("k_big_entity_rows"))) return rc;
     k_max_col<<<296, 256, 0, s>>>(col_len, p->N, maxc);
     if ((rc = launch_check("k_max_col"))) return rc;
   }
@@ -837,10 +920,9 @@ int plan_finish(const emg_plan *p, const int32_t *d_t2e, const int32_t *d_t2t, c
   const int32_t *ent_ptr = reinterpret_cast<const int32_t *>(plan + p->off_ent_ptr);
   Item *items = reinterpret_cast<Item *>(plan + p->off_item);
   uint32_t *ent_cnt = reinterpret_cast<uint32_t *>(plan + p->off_ent_cnt);
-  k_entity_rows<true><<<grid_for(p->n_ent, ROWS_WARPS), ROWS_WARPS * 32, 0, s>>>(
-      d_t2e, d_t2t, d_tetids, p->n_tets, p->n_edges, p->n_tris, ent_ptr, items, p->n_ent, nullptr, ent_cnt,
-      d_indptr, d_indices, d_status);
-  int rc = launch_check("k_entity_rows<fill>");
+  k_entity_indices<<<grid_for(p->n_ent, ROWS_WARPS), ROWS_WARPS * 32, 0, s>>>(
+      d_t2e, d_t2t, d_tetids, p->n_tets, p->n_edges, p->n_tris, ent_ptr, items, p->n_ent, ent_cnt, d_indptr, d_indices);
+  int rc = launch_check("k_entity_indices");
   if (rc) return rc;
   void *pidx = plan + p->off_pidx;
   if (p->value_layout != EMG_LAYOUT_BLOCK) {
@@ -849,7 +931,8 @@ int plan_finish(const emg_plan *p, const int32_t *d_t2e, const int32_t *d_t2t, c
         pidx, p->record_bytes == 4, d_status);
     return launch_check("k_chunk_contrib");
   }
-  k_chunk_blocks<<<grid_for(n_chunks(p->n_edges, p->n_tris), CC_WARPS), CC_WARPS * 32, 0, s>>>(
+  const int64_t block_ctas = (n_chunks(p->n_edges, p->n_tris) + CC_WARPS - 1) / CC_WARPS;
+  k_chunk_blocks<<<(int)(block_ctas < persistent_ctas(8) ? block_ctas : persistent_ctas(8)), CC_WARPS * 32, 0, s>>>(
       ent_ptr, items, ent_cnt, p->n_edges, p->n_tris, d_indptr, static_cast<uint32_t *>(pidx), d_status);
   if ((rc = launch_check("k_chunk_blocks"))) return rc;
   return write_chunk_desc(p, plan, d_indptr, s);
@@ -902,7 +985,7 @@ int plan_order(const emg_plan *p, void *d_plan, const double *nodes, int64_t nN,
   k_bbox_partial<<<BBOX_BLOCKS, 256, 0, s>>>(nodes, nN, part);
   int rc = launch_check("k_bbox_partial");
   if (rc) return rc;
-  k_bbox_final<<<1, 32, 0, s>>>(part, BBOX_BLOCKS, box);
+  k_bbox_final<<<1, 6 * 32, 0, s>>>(part, BBOX_BLOCKS, box);
   if ((rc = launch_check("k_bbox_final"))) return rc;
   k_chunk_keys<<<grid_for(n2, 256), 256, 0, s>>>(
       reinterpret_cast<const int32_t *>(plan + p->off_ent_ptr), reinterpret_cast<const Item *>(plan + p->off_item),
