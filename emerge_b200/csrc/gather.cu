@@ -507,43 +507,77 @@ __global__ void __launch_bounds__(BG_WARPS * 32, BG_CTAS)
 // frequency sweep: A_f = a_f K + b_f M (+ c_f P)
 // ---------------------------------------------------------------------------
 constexpr int SWEEP_MAX = 32;
+// CTAs per SM, oversubscribed: at 28.8M nonzeros and 12 frequencies 64 take 1,003
+// us, 8 1,033; one 16-byte access per element and 8 CTAs 1,181. Bound: HBM (6.5 TB/s).
+constexpr int SWEEP_CTAS = 64;
 struct SweepCoef {
   double c[SWEEP_MAX][6];
 };
 
-// Four elements per thread per pass: their loads are independent of the
-// previous pass's stores (restrict), so they are in flight together; the
-// arithmetic per value is unchanged.
-template <bool HASP>
+// Elements of a thread per access: two (32-byte loads and stores) where every
+// array is aligned to that and nnz is even, else one.
+template <int V>
+struct Elems {
+  double2 v[V];
+};
+
+template <int V>
+__device__ __forceinline__ Elems<V> ld_elems(const double2 *p) {
+  Elems<V> e;
+  if constexpr (V == 2)
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(e.v[0].x), "=d"(e.v[0].y), "=d"(e.v[1].x), "=d"(e.v[1].y)
+                 : "l"(p));
+  else
+    e.v[0] = __ldg(p);
+  return e;
+}
+
+template <int V>
+__device__ __forceinline__ void st_elems(double2 *p, const Elems<V> &e) {
+  if constexpr (V == 2)
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(e.v[0].x), "d"(e.v[0].y), "d"(e.v[1].x),
+                 "d"(e.v[1].y)
+                 : "memory");
+  else
+    *p = e.v[0];
+}
+
+// SWEEP_U accesses of K, M (and P) per thread per pass, all in flight before the
+// first output; the arithmetic per value is the same for all V.
+constexpr int SWEEP_U = 2;
+template <bool HASP, int V>
 __global__ void __launch_bounds__(256) k_form_sweep(const double2 *__restrict__ K, const double2 *__restrict__ M,
                                                     const double2 *__restrict__ P, int64_t nnz, SweepCoef cf, int nf,
                                                     double2 *__restrict__ out, int64_t stride) {
-  constexpr int U = 4;
-  const int64_t T = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < nnz; i0 += U * T) {
-    double2 k[U], m[U], p[U];
+  constexpr int U = SWEEP_U;
+  const int64_t T = (int64_t)gridDim.x * blockDim.x, n = nnz / V;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * T) {
+    Elems<V> k[U], m[U], p[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t i = i0 + u * T;
-      const bool in = i < nnz;
-      k[u] = in ? __ldg(K + i) : make_double2(0.0, 0.0);
-      m[u] = in ? __ldg(M + i) : make_double2(0.0, 0.0);
-      p[u] = (HASP && in) ? __ldg(P + i) : make_double2(0.0, 0.0);
+      const int64_t i = min(i0 + u * T, n - 1) * V;
+      k[u] = ld_elems<V>(K + i);
+      m[u] = ld_elems<V>(M + i);
+      if (HASP) p[u] = ld_elems<V>(P + i);
     }
     for (int f = 0; f < nf; ++f) {
       const double *c = cf.c[f];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int64_t i = i0 + u * T;
-        if (i >= nnz) break;
-        double2 o;
-        o.x = c[0] * k[u].x - c[1] * k[u].y + c[2] * m[u].x - c[3] * m[u].y;
-        o.y = c[0] * k[u].y + c[1] * k[u].x + c[2] * m[u].y + c[3] * m[u].x;
-        if (HASP) {
-          o.x += c[4] * p[u].x - c[5] * p[u].y;
-          o.y += c[4] * p[u].y + c[5] * p[u].x;
+        if (i >= n) break;
+        Elems<V> o;
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          o.v[q].x = c[0] * k[u].v[q].x - c[1] * k[u].v[q].y + c[2] * m[u].v[q].x - c[3] * m[u].v[q].y;
+          o.v[q].y = c[0] * k[u].v[q].y + c[1] * k[u].v[q].x + c[2] * m[u].v[q].y + c[3] * m[u].v[q].x;
+          if (HASP) {
+            o.v[q].x += c[4] * p[u].v[q].x - c[5] * p[u].v[q].y;
+            o.v[q].y += c[4] * p[u].v[q].y + c[5] * p[u].v[q].x;
+          }
         }
-        out[(int64_t)f * stride + i] = o;
+        st_elems<V>(out + (int64_t)f * stride + i * V, o);
       }
     }
   }
@@ -720,13 +754,17 @@ int launch_form_sweep(const void *d_K, const void *d_M, const void *d_P, int64_t
     SweepCoef c;
     memcpy(c.c, h_coef + (size_t)f0 * 6, (size_t)n * 6 * sizeof(double));
     double2 *o = static_cast<double2 *>(d_out) + (int64_t)f0 * out_stride;
-    const int g = persistent_ctas(8);  // oversubscribed: measured faster than one resident wave
-    if (d_P)
-      k_form_sweep<true><<<g, 256, 0, s>>>((const double2 *)d_K, (const double2 *)d_M, (const double2 *)d_P, nnz, c,
-                                           n, o, out_stride);
-    else
-      k_form_sweep<false><<<g, 256, 0, s>>>((const double2 *)d_K, (const double2 *)d_M, nullptr, nnz, c, n, o,
-                                            out_stride);
+    const int g = std::min(persistent_ctas(SWEEP_CTAS), grid_for(nnz, 256));
+    auto aligned = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 32 == 0; };
+    const bool two = nnz % 2 == 0 && out_stride % 2 == 0 && aligned(d_K) && aligned(d_M) && aligned(d_P) && aligned(o);
+#define EMG_FS(HASP, V) \
+  k_form_sweep<HASP, V><<<g, 256, 0, s>>>((const double2 *)d_K, (const double2 *)d_M, (const double2 *)d_P, nnz, c, n, o, out_stride)
+    if (d_P) {
+      if (two) EMG_FS(true, 2); else EMG_FS(true, 1);
+    } else {
+      if (two) EMG_FS(false, 2); else EMG_FS(false, 1);
+    }
+#undef EMG_FS
     int rc = launch_check("k_form_sweep");
     if (rc) return rc;
   }
