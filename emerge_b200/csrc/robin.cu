@@ -313,10 +313,16 @@ __global__ void k_pad_keys(uint64_t *keys, int64_t from, int64_t n_keys) {
   if (k < n_keys) keys[k] = ~0ull;
 }
 
-// A[p] += gamma * (sum of the slots of target p, in slot order); one thread
-// per sorted slot, the first slot of each target sums its run
-__global__ void k_robin_apply(const uint64_t *keys, int64_t n_slots, const double2 *vals, double gr, double gi,
-                              double2 *A, int64_t nnz) {
+// A_f[p] += gamma_f * (sum of the slots of target p, in slot order) for nf arrays
+// A_f = A + f * stride; one thread per sorted slot, the first slot of each
+// target sums its run, once for all f
+constexpr int APPLY_MAX = 64;
+struct Gammas {
+  double g[APPLY_MAX][2];
+};
+
+__global__ void k_robin_apply(const uint64_t *keys, int64_t n_slots, const double2 *vals, const Gammas gamma, int nf,
+                              double2 *A, int64_t stride, int64_t nnz) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_slots) return;
   const uint64_t key = keys[i];
@@ -334,10 +340,29 @@ __global__ void k_robin_apply(const uint64_t *keys, int64_t n_slots, const doubl
     sr += v.x;
     si += v.y;
   }
-  double2 a = A[p];
-  a.x += gr * sr - gi * si;
-  a.y += gr * si + gi * sr;
-  A[p] = a;
+  double2 *o = A + p;
+#pragma unroll 4
+  for (int f = 0; f < nf; ++f) {
+    const double gr = gamma.g[f][0], gi = gamma.g[f][1];
+    double2 a = o[f * stride];
+    a.x += gr * sr - gi * si;
+    a.y += gr * si + gi * sr;
+    o[f * stride] = a;
+  }
+}
+
+int launch_apply(const uint64_t *keys, int64_t n_slots, const void *vals, const double *h_gamma, int nf, void *A,
+                 int64_t stride, int64_t nnz, cudaStream_t s) {
+  for (int f0 = 0; f0 < nf; f0 += APPLY_MAX) {
+    const int n = nf - f0 < APPLY_MAX ? nf - f0 : APPLY_MAX;
+    Gammas g;
+    memcpy(g.g, h_gamma + 2 * (size_t)f0, (size_t)n * 2 * sizeof(double));
+    k_robin_apply<<<grid_for(n_slots, 256), 256, 0, s>>>(keys, n_slots, static_cast<const double2 *>(vals), g, n,
+                                                         static_cast<double2 *>(A) + (int64_t)f0 * stride, stride, nnz);
+    const int rc = launch_check("k_robin_apply");
+    if (rc) return rc;
+  }
+  return EMG_OK;
 }
 
 }  // namespace
@@ -428,10 +453,17 @@ int emg_robin_apply(const emg_robin *r, const uint64_t *d_keys, const void *d_va
   if (!r) return fail(EMG_EINVAL, "null robin descriptor");
   if (r->n_btris == 0) return EMG_OK;
   if (!d_keys || !d_values || !d_A) return fail(EMG_EINVAL, "null pointer");
-  k_robin_apply<<<grid_for(r->n_slots, 256), 256, 0, S(stream)>>>(
-      d_keys, r->n_slots, static_cast<const double2 *>(d_values), gamma_re, gamma_im, static_cast<double2 *>(d_A),
-      nnz);
-  return launch_check("k_robin_apply");
+  const double g[2] = {gamma_re, gamma_im};
+  return launch_apply(d_keys, r->n_slots, d_values, g, 1, d_A, nnz, nnz, S(stream));
+}
+
+int emg_robin_apply_sweep(const emg_robin *r, const uint64_t *d_keys, const void *d_values, const double *h_gamma, int nf,
+                          void *d_A, int64_t stride, int64_t nnz, emg_stream_t stream) {
+  if (!r) return fail(EMG_EINVAL, "null robin descriptor");
+  if (nf < 0 || stride < nnz) return fail(EMG_EINVAL, "bad frequency count or stride");
+  if (r->n_btris == 0 || nf == 0) return EMG_OK;
+  if (!d_keys || !d_values || !h_gamma || !d_A) return fail(EMG_EINVAL, "null pointer");
+  return launch_apply(d_keys, r->n_slots, d_values, h_gamma, nf, d_A, stride, nnz, S(stream));
 }
 
 int emg_robin_force(const emg_robin *r, const double *d_nodes, int64_t n_nodes, const int32_t *d_tris,
@@ -455,10 +487,8 @@ int emg_robin_force(const emg_robin *r, const double *d_nodes, int64_t n_nodes, 
     if ((rc = launch_check("k_pad_keys"))) return rc;
   }
   if ((rc = sort_u64(d_fkeys, r->n_fkeys, s))) return rc;
-  k_robin_apply<<<grid_for(r->n_fslots, 256), 256, 0, s>>>(d_fkeys, r->n_fslots,
-                                                           static_cast<const double2 *>(d_fvalues), 1.0, 0.0,
-                                                           static_cast<double2 *>(d_b), N);
-  return launch_check("k_robin_apply");
+  const double one[2] = {1.0, 0.0};
+  return launch_apply(d_fkeys, r->n_fslots, d_fvalues, one, 1, d_b, N, N, s);
 }
 
 }  // extern "C"

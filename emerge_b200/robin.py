@@ -172,6 +172,17 @@ class RobinTerm:
                                         g.imag, L.ptr(A), self.cmap.nnz, L.stream_handle(self.cmap.device)))
         return A
 
+    def apply_sweep(self, A: torch.Tensor, gamma) -> torch.Tensor:
+        """A[f, p] += gamma[f] * (the term at p) for every row of A (complex128
+        [nf, nnz], contiguous, device), in one launch; stream-ordered."""
+        g = np.ascontiguousarray(gamma, dtype=np.complex128).ravel()
+        if A.dtype != torch.complex128 or A.shape != (g.size, self.cmap.nnz) or not A.is_contiguous():
+            raise ValueError("A must be a contiguous complex128 tensor of (nf, nnz) values")
+        L.check(L.lib().emg_robin_apply_sweep(L.ctypes.byref(self.desc), L.ptr(self.d_keys), L.ptr(self.d_vals),
+                                              g.ctypes.data_as(L.ctypes.POINTER(L.ctypes.c_double)), int(g.size), L.ptr(A),
+                                              self.cmap.nnz, self.cmap.nnz, L.stream_handle(self.cmap.device)))
+        return A
+
     def to_device(self, gamma: complex = 1.0) -> torch.Tensor:
         """gamma times the term on A's pattern (complex128 [nnz], zeros off the
         boundary), e.g. the P of a frequency sweep."""

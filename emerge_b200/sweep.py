@@ -109,9 +109,12 @@ class FrequencySweep:
             g = np.asarray(robin_gamma, dtype=np.complex128).reshape(nf, -1)
             if g.shape[1] != len(self.robin):
                 raise ValueError(f"robin_gamma needs {len(self.robin)} column(s)")
-            for i in range(nf):
-                for j, r in enumerate(self.robin):
-                    r.apply(out[i], complex(g[i, j]))
+            for j, r in enumerate(self.robin):
+                if hasattr(r, "apply_sweep"):
+                    r.apply_sweep(out, g[:, j])
+                else:
+                    for i in range(nf):
+                        r.apply(out[i], complex(g[i, j]))
         elif robin_gamma is not None:
             raise ValueError("robin_gamma given but the sweep has no boundary term")
         return out

@@ -420,6 +420,12 @@ int emg_abc2_build(const emg_robin *robin, const double *d_nodes, int64_t n_node
 int emg_robin_apply(const emg_robin *robin, const uint64_t *d_keys, const void *d_values, double gamma_re,
                     double gamma_im, void *d_A, int64_t nnz, emg_stream_t stream);
 
+/* The same for nf arrays at d_A + f * stride (complex128 elements, stride >=
+ * nnz) with h_gamma[f] = (re, im) each, as emg_form_sweep writes them: the
+ * slots of a position are summed once for all of them. */
+int emg_robin_apply_sweep(const emg_robin *robin, const uint64_t *d_keys, const void *d_values, const double *h_gamma,
+                          int nf, void *d_A, int64_t stride, int64_t nnz, emg_stream_t stream);
+
 /* Port forcing vector: d_b[N] (complex128) += the boundary triangles'
  * ned2_tri_force entries (robinbc.py:220-313, assemble_robin_bc_bvec
  * :405-433) for the incident field d_U (complex128 [3][6][n_btris]: component,
