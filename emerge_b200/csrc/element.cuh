@@ -832,10 +832,10 @@ __device__ __forceinline__ void do_row_block(const Tensors<KIND, R> &T, const R 
 
 template <int FORM, int KIND, typename R, int... Is>
 __device__ __forceinline__ void all_rows_block(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
-                                               const CR<R> &cM, uint64_t inv, bool active, int ia,
+                                               const CR<R> &cM, uint64_t inv, bool active, int ia, unsigned rows,
                                                typename StoreT<R>::T *stage, typename StoreT<R>::T *out,
                                                std::integer_sequence<int, Is...>) {
-  (do_row_block<FORM, KIND, R, Is>(T, mu, sig, cK, cM, inv, active, ia, stage, out), ...);
+  ((rows >> Is & 1u ? do_row_block<FORM, KIND, R, Is>(T, mu, sig, cK, cM, inv, active, ia, stage, out) : (void)0), ...);
 }
 
 // LAYOUT 0: the reference's COO block [ia][a][b] (400 values, each entry
@@ -848,7 +848,7 @@ __device__ __forceinline__ void all_rows_block(const Tensors<KIND, R> &T, const 
 // TK: the tensors' form. Returns whether any tet of the warp needs the
 // antisymmetric pass.
 template <int FORM, int KIND, int LAYOUT, int TK>
-__device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, unsigned char *stage_raw) {
+__device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, unsigned rows, unsigned char *stage_raw) {
   using R = typename FormReal<FORM>::T;
   using ST = typename StoreT<R>::T;
   constexpr int LPT = lanes_per_tet(TK);
@@ -954,7 +954,7 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
   if constexpr (LAYOUT == 0) {
     all_rows<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out, std::make_integer_sequence<int, 20>{});
   } else if constexpr (LAYOUT == 2) {
-    all_rows_block<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
+    all_rows_block<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, rows, stage, out,
                                   std::make_integer_sequence<int, 10>{});
   } else {
     all_rows_packed<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
@@ -963,12 +963,27 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
   return TK == KIND_PAIR_FULL && __any_sync(0xffffffffu, asym);
 }
 
+// rows: bit i set to write block row i (block layout; the others write all rows)
 template <int FORM, int KIND, int LAYOUT>
-__device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsigned char *stage_raw) {
+__device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsigned rows, unsigned char *stage_raw) {
   constexpr int TK = tensor_kind(FORM, KIND);
-  const bool asym = element_pass<FORM, KIND, LAYOUT, TK>(a, ia0, stage_raw);
+  const bool asym = element_pass<FORM, KIND, LAYOUT, TK>(a, ia0, rows, stage_raw);
   if constexpr (TK == KIND_PAIR_FULL)
-    if (asym) element_pass<FORM, KIND, LAYOUT, KIND_PAIR_ANTI>(a, ia0, stage_raw);
+    if (asym) element_pass<FORM, KIND, LAYOUT, KIND_PAIR_ANTI>(a, ia0, rows, stage_raw);
+}
+
+// A mesh that leaves most of the GPU idle: its tets are gone through by several
+// CTAs, blockIdx.y of n_parts, each of which forms the geometry and moments again
+// but only some of the block rows (row i has 10 - i blocks). The time of such a
+// launch is that of one tet: 4,950 tets mixed 20.5 -> 12.3 us and FP64 28.7 -> 20.5
+// in five parts, 12,960 mixed 21.5 -> 14.4 in five and FP64 28.7 -> 26.6 in two.
+// More parts than fit at once would put the repeated part into a second wave.
+constexpr unsigned ALL_ROWS = 0x3ffu;
+__device__ __forceinline__ unsigned part_rows(int part, int n_parts) {
+  if (n_parts == 2) return part ? 0x3f8u : 0x007u;                                  // 27 and 28 blocks
+  if (n_parts == 3) return part == 0 ? 0x003u : (part == 1 ? 0x10cu : 0x2f0u);      // 19, 17, 19
+  if (n_parts == 5) return (1u << part) | (1u << (9 - part));                       // 11 each
+  return ALL_ROWS;
 }
 
 // CTAs per SM the compiler must fit. Measured on the 2.01M-tet box: the
@@ -990,7 +1005,8 @@ __host__ __device__ constexpr int elem_tets() {
 template <int FORM, int KIND, int LAYOUT>
 __global__ void __launch_bounds__(ELEM_THREADS, elem_min_blocks<FORM, KIND>()) k_element(ElemArgs a) {
   extern __shared__ __align__(16) unsigned char stage_raw[];
-  element_cta<FORM, KIND, LAYOUT>(a, (int64_t)blockIdx.x * elem_tets<FORM, KIND>(), stage_raw);
+  element_cta<FORM, KIND, LAYOUT>(a, (int64_t)blockIdx.x * elem_tets<FORM, KIND>(), part_rows(blockIdx.y, gridDim.y),
+                                  stage_raw);
 }
 
 // Several jobs (meshes, materials, coefficients, outputs) in one launch of
@@ -1008,7 +1024,13 @@ __global__ void __launch_bounds__(ELEM_THREADS, elem_min_blocks<FORM, KIND>())
     else hi = mid - 1;
   }
   if (n_jobs <= 0 || b >= cta_start[n_jobs]) return;
-  element_cta<FORM, KIND, LAYOUT>(jobs[lo], (b - cta_start[lo]) * elem_tets<FORM, KIND>(), stage_raw);
+  element_cta<FORM, KIND, LAYOUT>(jobs[lo], (b - cta_start[lo]) * elem_tets<FORM, KIND>(), ALL_ROWS, stage_raw);
+}
+
+// CTAs that share an SM, by registers and stage
+template <int FORM, int KIND>
+constexpr int elem_ctas_per_sm() {
+  return FORM == FORM_REF32 ? (KIND == EMG_MAT_ISO ? 5 : (KIND == EMG_MAT_DIAG ? 3 : 2)) : 2;
 }
 
 template <int FORM, int KIND, int LAYOUT>
@@ -1028,7 +1050,12 @@ int launch_element_t(const ElemArgs &a, cudaStream_t s) {
     if (dev < 64) configured[dev] = true;
   }
   if (a.nA == 0) return EMG_OK;
-  k_element<FORM, KIND, LAYOUT><<<grid_for(a.nA, elem_tets<FORM, KIND>()), ELEM_THREADS, smem, s>>>(a);
+  const int ctas = grid_for(a.nA, elem_tets<FORM, KIND>());
+  int parts = 1;
+  if (LAYOUT == 2)  // the most parts that still fit the GPU at once
+    for (int p : {2, 3, 5})
+      if ((int64_t)ctas * p <= persistent_ctas(elem_ctas_per_sm<FORM, KIND>())) parts = p;
+  k_element<FORM, KIND, LAYOUT><<<dim3(ctas, parts), ELEM_THREADS, smem, s>>>(a);
   return launch_check("k_element");
 }
 
