@@ -25,9 +25,10 @@
 //
 // Every form writes one of three layouts (element_cta): the reference's COO
 // block value[ia*400 + 20*a + b], the packed canonical upper triangle
-// [ia][210], or the entity-pair blocks [ia][220] of the assembly path. One row
-// of the block at a time is staged in shared memory and the warp writes its
-// 32 tets' rows as contiguous runs.
+// [ia][210], or the entity-pair blocks [ia][220] of the assembly path. Of the
+// first two, one row at a time is staged in shared memory and the warp writes its
+// tets' rows as contiguous runs; the blocks are stored straight from registers
+// where a lane holds whole values.
 #pragma once
 #include "common.cuh"
 
@@ -716,15 +717,11 @@ __device__ __forceinline__ void all_rows(const Tensors<KIND, R> &T, const R *mu,
 // 20 - X upper-triangle entries) is staged in shared memory and the warp
 // writes its 32 row segments as contiguous runs.
 template <int x, int y, int FORM, int KIND, typename R>
-__device__ __forceinline__ void compute_store_packed(const Tensors<KIND, R> &T, const R *mu, double sig,
-                                                     const CR<R> &cK, const CR<R> &cM, uint64_t inv,
-                                                     typename StoreT<R>::T *row) {
-  using ST = typename StoreT<R>::T;
-  ST v;
-  if constexpr (KIND >= KIND_PAIR) {
-    reinterpret_cast<R *>(row + (y - x))[threadIdx.x & 1] = pair_value<x, y, FORM, KIND, R>(T, mu, sig, inv);
-    return;
-  } else if constexpr (KIND == EMG_MAT_ISO) {
+__device__ __forceinline__ typename StoreT<R>::T packed_value(const Tensors<KIND, R> &T, const R *mu, double sig,
+                                                              const CR<R> &cK, const CR<R> &cM, uint64_t inv) {
+  static_assert(KIND < KIND_PAIR, "a pair's lanes hold half a value each");
+  typename StoreT<R>::T v;
+  if constexpr (KIND == EMG_MAT_ISO) {
     R k0, m0;
     entry<x, y, FORM, KIND, R>(T, mu, sig, k0, m0);
     v.x = cfma(cK.re, k0, cmul_rn(cM.re, m0));
@@ -744,7 +741,17 @@ __device__ __forceinline__ void compute_store_packed(const Tensors<KIND, R> &T, 
     v.x = cfma(cK.re, k.re, cfma(-cK.im, k.im, cfma(cM.re, m.re, cmul_rn(-cM.im, m.im))));
     v.y = cfma(cK.re, k.im, cfma(cK.im, k.re, cfma(cM.re, m.im, cmul_rn(cM.im, m.re))));
   }
-  row[y - x] = v;
+  return v;
+}
+
+template <int x, int y, int FORM, int KIND, typename R>
+__device__ __forceinline__ void compute_store_packed(const Tensors<KIND, R> &T, const R *mu, double sig,
+                                                     const CR<R> &cK, const CR<R> &cM, uint64_t inv,
+                                                     typename StoreT<R>::T *row) {
+  if constexpr (KIND >= KIND_PAIR)
+    reinterpret_cast<R *>(row + (y - x))[threadIdx.x & 1] = pair_value<x, y, FORM, KIND, R>(T, mu, sig, inv);
+  else
+    row[y - x] = packed_value<x, y, FORM, KIND, R>(T, mu, sig, cK, cM, inv);
 }
 
 template <int x, int FORM, int KIND, typename R, int... Ds>
@@ -784,50 +791,142 @@ __device__ __forceinline__ void all_rows_packed(const Tensors<KIND, R> &T, const
 }
 
 // ---- entity-pair block layout: value[ia*220 + 4*block_index(i, j) + k] for
-// canonical entities i <= j. Block row i (its 10 - i blocks, 4 values each)
-// is staged in shared memory and the warp writes its 32 block rows as
-// contiguous runs. Each value is the packed layout's (min, max) entry.
+// canonical entities i <= j. Each value is the packed layout's (min, max) entry.
+// wide: values aligned to 32 bytes, written a whole sector at a time; others are
+// written one by one.
+//
+// A lane that owns its tet stores the values straight from registers, a sector per
+// instruction: half a complex128 block or a complex64 block. The stores need no
+// answer and drain beside the arithmetic. Staged in shared memory and written by
+// the warp as runs of up to 640 bytes, rows and write-back took turns in the eight
+// warps that the registers leave an SM. 1.008M tets: isotropic FP64 779 -> 640 us
+// (3.55 GB; 447 without its stores), exact isotropic 619. The mixed form, 367 ->
+// 362, is bound by these writes: 82 without them, and tets 1,760 bytes apart take
+// them at 4.9 TB/s where a fill reaches 7.3. Tiles of 4 to 32 tets per block
+// would be written faster (mixed 314 to 332) but scatter what the gather reads:
+// 1,426 -> 2,326 us with the tets in random order.
+__device__ __forceinline__ void store_half(double2 *o, double2 v0, double2 v1, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(o), "d"(v0.x), "d"(v0.y), "d"(v1.x), "d"(v1.y)
+                 : "memory");
+  } else {
+    o[0] = v0;
+    o[1] = v1;
+  }
+}
+
+__device__ __forceinline__ void store_block(float2 *o, float2 v0, float2 v1, float2 v2, float2 v3, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o), "f"(v0.x), "f"(v0.y),
+                 "f"(v1.x), "f"(v1.y), "f"(v2.x), "f"(v2.y), "f"(v3.x), "f"(v3.y)
+                 : "memory");
+  } else {
+    o[0] = v0;
+    o[1] = v1;
+    o[2] = v2;
+    o[3] = v3;
+  }
+}
+
+// A block row's values as one lane forms them, in the order that it stores them:
+// FP64 the first DoF's entries of all blocks, then the second's (the packed
+// triangle's row order); FP32 block by block.
+template <int FORM, int KIND, typename R>
+struct BlockRow {
+  using ST = typename StoreT<R>::T;
+  const Tensors<KIND, R> &T;
+  const R *mu;
+  const double sig;
+  const CR<R> &cK, &cM;
+  const uint64_t inv;
+  const bool wide;
+
+  template <int x, int y>
+  __device__ __forceinline__ ST value() const {
+    return packed_value<(x < y ? x : y), (x < y ? y : x), FORM, KIND, R>(T, mu, sig, cK, cM, inv);
+  }
+  // entries (x, first DoF of entity j) and (x, second DoF of j)
+  template <int x, int j>
+  __device__ __forceinline__ void half(ST *o) const {
+    const ST v0 = value<x, ent_dof1(j)>(), v1 = value<x, ent_dof2(j)>();
+    store_half(o, v0, v1, wide);
+  }
+  template <int i, int j>
+  __device__ __forceinline__ void block(ST *o) const {
+    const ST v0 = value<ent_dof1(i), ent_dof1(j)>(), v1 = value<ent_dof1(i), ent_dof2(j)>();
+    const ST v2 = value<ent_dof2(i), ent_dof1(j)>(), v3 = value<ent_dof2(i), ent_dof2(j)>();
+    store_block(o, v0, v1, v2, v3, wide);
+  }
+  template <int i, int... Js>
+  __device__ __forceinline__ void store(ST *row, std::integer_sequence<int, Js...>) const {
+    if constexpr (sizeof(R) == 4) {
+      (block<i, i + Js>(row + 4 * Js), ...);
+    } else {
+      (half<ent_dof1(i), i + Js>(row + 4 * Js), ...);
+      (half<ent_dof2(i), i + Js>(row + 4 * Js + 2), ...);
+    }
+  }
+};
+
+// A pair's lanes hold half a value each, so their row is staged, one tet's values
+// an odd number apart, and the warp writes its 16 tets' rows, for diagonal tensors
+// two values at a time: 1.008M tets, one 1,120 us, two 1,060, exchanged by a shuffle
+// and stored by the lanes 1,100. Full tensors leave no registers for it (504k tets,
+// one 690 us, two 799, by the lanes 904).
 template <int x, int y, int FORM, int KIND, typename R>
-__device__ __forceinline__ void compute_store_any(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
-                                                  const CR<R> &cM, uint64_t inv, typename StoreT<R>::T *dst) {
-  constexpr int lo = x < y ? x : y, hi = x < y ? y : x;
-  compute_store_packed<lo, hi, FORM, KIND, R>(T, mu, sig, cK, cM, inv, dst - (hi - lo));
+__device__ __forceinline__ void stage_half_value(const Tensors<KIND, R> &T, const R *mu, double sig, uint64_t inv,
+                                                 double2 *dst) {
+  reinterpret_cast<R *>(dst)[threadIdx.x & 1] =
+      pair_value<(x < y ? x : y), (x < y ? y : x), FORM, KIND, R>(T, mu, sig, inv);
 }
 
 template <int i, int FORM, int KIND, typename R, int... Js>
-__device__ __forceinline__ void compute_block_row(const Tensors<KIND, R> &T, const R *mu, double sig,
-                                                  const CR<R> &cK, const CR<R> &cM, uint64_t inv,
-                                                  typename StoreT<R>::T *row, std::integer_sequence<int, Js...>) {
-  // the first DoF's entries of the block row, then the second's (row order of the packed triangle)
-  ((compute_store_any<ent_dof1(i), ent_dof1(i + Js), FORM, KIND, R>(T, mu, sig, cK, cM, inv, row + 4 * Js + 0),
-    compute_store_any<ent_dof1(i), ent_dof2(i + Js), FORM, KIND, R>(T, mu, sig, cK, cM, inv, row + 4 * Js + 1)),
+__device__ __forceinline__ void stage_block_row(const Tensors<KIND, R> &T, const R *mu, double sig, uint64_t inv,
+                                                double2 *row, std::integer_sequence<int, Js...>) {
+  ((stage_half_value<ent_dof1(i), ent_dof1(i + Js), FORM, KIND, R>(T, mu, sig, inv, row + 4 * Js + 0),
+    stage_half_value<ent_dof1(i), ent_dof2(i + Js), FORM, KIND, R>(T, mu, sig, inv, row + 4 * Js + 1)),
    ...);
-  ((compute_store_any<ent_dof2(i), ent_dof1(i + Js), FORM, KIND, R>(T, mu, sig, cK, cM, inv, row + 4 * Js + 2),
-    compute_store_any<ent_dof2(i), ent_dof2(i + Js), FORM, KIND, R>(T, mu, sig, cK, cM, inv, row + 4 * Js + 3)),
+  ((stage_half_value<ent_dof2(i), ent_dof1(i + Js), FORM, KIND, R>(T, mu, sig, inv, row + 4 * Js + 2),
+    stage_half_value<ent_dof2(i), ent_dof2(i + Js), FORM, KIND, R>(T, mu, sig, inv, row + 4 * Js + 3)),
    ...);
 }
 
 template <int FORM, int KIND, typename R, int I>
 __device__ __forceinline__ void do_row_block(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
-                                             const CR<R> &cM, uint64_t inv, bool active, int ia,
+                                             const CR<R> &cM, uint64_t inv, bool active, int ia, bool wide,
                                              typename StoreT<R>::T *stage, typename StoreT<R>::T *out) {
-  constexpr int W = 4 * (10 - I), LPT = lanes_per_tet(KIND);
-  const int lane = threadIdx.x & 31;
-  if (active)
-    compute_block_row<I, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane / LPT * (W | 1),
+  if constexpr (KIND < KIND_PAIR) {
+    if (active)
+      BlockRow<FORM, KIND, R>{T, mu, sig, cK, cM, inv, wide}.template store<I>(
+          out + (int64_t)ia * kBlockValues + 4 * block_index(I, I), std::make_integer_sequence<int, 10 - I>{});
+    __syncwarp();  // the compiler would otherwise form products of later rows ahead, and spill them
+  } else {
+    // V values at a time
+    constexpr int W = 4 * (10 - I), LPT = lanes_per_tet(KIND), V = KIND == KIND_PAIR ? 2 : 1, ROUNDS = W / LPT / V;
+    static_assert(W % (LPT * V) == 0, "whole rounds of the warp");
+    const int lane = threadIdx.x & 31;
+    if (active)
+      stage_block_row<I, FORM, KIND, R>(T, mu, sig, inv, stage + lane / LPT * (W | 1),
                                         std::make_integer_sequence<int, 10 - I>{});
-  // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
-  const unsigned act = __ballot_sync(0xffffffffu, active);
-  const int64_t ia_w = (int64_t)ia - lane / LPT;
-  __syncwarp();
+    // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    const int64_t ia_w = (int64_t)ia - lane / LPT;
+    __syncwarp();
 #pragma unroll 2
-  for (int it = 0; it < W / LPT; ++it) {
-    const int e = it * 32 + lane;
-    const int r = e / W, c = e - r * W;
-    if ((act >> (r * LPT)) & 1u)
-      put<KIND>(out + (ia_w + r) * kBlockValues + 4 * block_index(I, I) + c, stage[r * (W | 1) + c]);
+    for (int it = 0; it < ROUNDS; ++it) {
+      const int e = it * 32 + lane;
+      const int r = e / (W / V), c = V * (e - r * (W / V));
+      if ((act >> (r * LPT)) & 1u) {
+        double2 *o = out + (ia_w + r) * kBlockValues + 4 * block_index(I, I) + c;
+        const double2 *v = stage + r * (W | 1) + c;
+        if constexpr (V == 2)
+          store_half(o, v[0], v[1], wide);
+        else
+          put<KIND>(o, v[0]);
+      }
+    }
+    __syncwarp();
   }
-  __syncwarp();
 }
 
 template <int FORM, int KIND, typename R, int... Is>
@@ -835,7 +934,17 @@ __device__ __forceinline__ void all_rows_block(const Tensors<KIND, R> &T, const 
                                                const CR<R> &cM, uint64_t inv, bool active, int ia, unsigned rows,
                                                typename StoreT<R>::T *stage, typename StoreT<R>::T *out,
                                                std::integer_sequence<int, Is...>) {
-  ((rows >> Is & 1u ? do_row_block<FORM, KIND, R, Is>(T, mu, sig, cK, cM, inv, active, ia, stage, out) : (void)0), ...);
+  const bool wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+  ((rows >> Is & 1u ? do_row_block<FORM, KIND, R, Is>(T, mu, sig, cK, cM, inv, active, ia, wide, stage, out)
+                    : (void)0),
+   ...);
+}
+
+// staged values per tet: the longest row, its stride odd, so that the lanes' stores
+// of one value position fall in distinct shared-memory bank groups
+template <int LAYOUT, int TK>
+__host__ __device__ constexpr int stage_values() {
+  return LAYOUT != 2 ? 21 : (TK >= KIND_PAIR ? 41 : 0);
 }
 
 // LAYOUT 0: the reference's COO block [ia][a][b] (400 values, each entry
@@ -852,9 +961,7 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
   using R = typename FormReal<FORM>::T;
   using ST = typename StoreT<R>::T;
   constexpr int LPT = lanes_per_tet(TK);
-  // values per tet: a row's stride is odd (in values), so the lanes' stores of
-  // one value position fall in distinct shared-memory bank groups
-  constexpr int STAGE = LAYOUT == 2 ? 41 : 21;
+  constexpr int STAGE = stage_values<LAYOUT, TK>();
   ST *stage = reinterpret_cast<ST *>(stage_raw) + (threadIdx.x >> 5) * (32 / LPT * STAGE);
   ST *out = reinterpret_cast<ST *>(a.out);
   const int64_t ia64 = ia0 + threadIdx.x / LPT;
@@ -955,7 +1062,7 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
     all_rows<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out, std::make_integer_sequence<int, 20>{});
   } else if constexpr (LAYOUT == 2) {
     all_rows_block<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, rows, stage, out,
-                                  std::make_integer_sequence<int, 10>{});
+                                std::make_integer_sequence<int, 10>{});
   } else {
     all_rows_packed<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
                                    std::make_integer_sequence<int, 20>{});
@@ -986,11 +1093,10 @@ __device__ __forceinline__ unsigned part_rows(int part, int n_parts) {
   return ALL_ROWS;
 }
 
-// CTAs per SM the compiler must fit. Measured on the 2.01M-tet box: the
-// isotropic FP64 forms at their natural 242-255 registers (two CTAs) beat every cap (a
-// three-CTA cap: 1.84 -> 3.68 ms, 1.9 KB of spills); the mixed form needs 88-254
-// registers with no cap (five CTAs per SM for the isotropic instance, set by
-// its 42 KB stage as much as by registers).
+// CTAs per SM the compiler must fit. The isotropic FP64 forms at their natural
+// 232-255 registers (two CTAs) beat every cap (three CTAs, 2.01M tets: 1.84 ->
+// 3.68 ms, 1.9 KB of spills); the mixed form takes 90-254 (five CTAs per SM for the
+// isotropic instance; held to six or seven, 1.008M tets: 362 -> 375 / 385 us).
 template <int FORM, int KIND>
 constexpr int elem_min_blocks() {
   return 1;
@@ -1036,7 +1142,8 @@ constexpr int elem_ctas_per_sm() {
 template <int FORM, int KIND, int LAYOUT>
 int launch_element_t(const ElemArgs &a, cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
-  constexpr size_t smem = (size_t)elem_tets<FORM, KIND>() * (LAYOUT == 2 ? 41 : 21) * sizeof(ST);
+  constexpr size_t smem =
+      (size_t)elem_tets<FORM, KIND>() * stage_values<LAYOUT, tensor_kind(FORM, KIND)>() * sizeof(ST);
   static_assert(elem_tets<FORM, KIND>() == elem_tets_per_cta(FORM, KIND), "the host's table of CTAs");
   // the attribute belongs to the current device: set once per device (benign
   // race: every thread that gets here sets the same value)
@@ -1063,7 +1170,8 @@ template <int FORM, int KIND, int LAYOUT>
 int launch_element_batch_t(const ElemArgs *d_jobs, const int64_t *d_cta_start, int n_jobs, int64_t total_ctas,
                            cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
-  constexpr size_t smem = (size_t)elem_tets<FORM, KIND>() * (LAYOUT == 2 ? 41 : 21) * sizeof(ST);  // element_cta's stage
+  constexpr size_t smem =  // element_cta's stage
+      (size_t)elem_tets<FORM, KIND>() * stage_values<LAYOUT, tensor_kind(FORM, KIND)>() * sizeof(ST);
   static bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
