@@ -28,7 +28,8 @@ EXPORTS = (
     "emg_robin_init", "emg_robin_build", "emg_abc2_build", "emg_robin_apply", "emg_robin_apply_sweep", "emg_robin_force",
     "emg_robin_build_dofs", "emg_csc_lookup", "emg_csc_shift",
     "emg_select_init", "emg_select_build", "emg_select_finish", "emg_select_values", "emg_ned2_interp",
-    "emg_port_overlap", "emg_sparse_solve", "emg_coo_init", "emg_coo_rowcol", "emg_coo_build", "emg_coo_finish", "emg_coo_gather",
+    "emg_port_overlap", "emg_sparse_solve", "emg_coo_init", "emg_coo_rowcol", "emg_coo_build", "emg_coo_finish",
+    "emg_coo_build_blocks", "emg_coo_finish_blocks", "emg_coo_gather",
     "emg_leg2_element",
 )
 
@@ -165,6 +166,8 @@ def lib():
     L.emg_coo_rowcol.argtypes = [_P, ctypes.c_int, _I64, _P, _P, _P]
     L.emg_coo_build.argtypes = [ctypes.POINTER(CooMap), _P, _P, _P, _P, _P, _P, _P]
     L.emg_coo_finish.argtypes = [ctypes.POINTER(CooMap), _P, _P, _P, _P, _P, _P, _P]
+    L.emg_coo_build_blocks.argtypes = [ctypes.POINTER(CooMap), _P, ctypes.c_int, _P, _P, _P, _P, _P]
+    L.emg_coo_finish_blocks.argtypes = [ctypes.POINTER(CooMap), _P, ctypes.c_int, _P, _P, _P, _P, _P, _P]
     L.emg_coo_gather.argtypes = [ctypes.POINTER(CooMap), _P, _P, ctypes.c_int, ctypes.c_int, _P, _P, _P]
     L.emg_leg2_element.argtypes = [_P, _I64, _P, _I64, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P, _P, _P]
     L.emg_robin_force.argtypes = [ctypes.POINTER(Robin), _P, _I64, _P, _P, _I64, _I64, _P, _P, _P, _P, _P, _I64, _P,
@@ -177,7 +180,8 @@ def lib():
                  "emg_robin_init", "emg_robin_build", "emg_abc2_build",
                  "emg_robin_apply", "emg_robin_apply_sweep", "emg_robin_force", "emg_select_init", "emg_select_build", "emg_select_finish",
                  "emg_select_values", "emg_ned2_interp", "emg_port_overlap", "emg_sparse_solve", "emg_coo_init", "emg_coo_rowcol",
-                 "emg_coo_build", "emg_coo_finish", "emg_coo_gather", "emg_leg2_element", "emg_plan_set_value_layout",
+                 "emg_coo_build", "emg_coo_finish", "emg_coo_build_blocks", "emg_coo_finish_blocks", "emg_coo_gather",
+                 "emg_leg2_element", "emg_plan_set_value_layout",
                  "emg_robin_build_dofs", "emg_csc_lookup", "emg_csc_shift"):
         getattr(L, name).restype = ctypes.c_int
     _lib = L

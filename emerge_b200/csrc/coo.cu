@@ -6,30 +6,71 @@
 // Pattern: slots counted per column, scattered into column buckets, each
 // bucket sorted by (row, slot) -- a fixed order, whatever order the scatter
 // left them in -- and its distinct rows become the column's entries; the value
-// of an entry is the sum of its slots in that order.
+// of an entry is the sum of its slots in that order. Slots that are the D x D blocks
+// of elements are counted and scattered as the D columns of each element, and
+// their rows read from the elements' DoFs.
 #include "common.cuh"
 
 namespace emg {
 namespace {
 
-__global__ void k_coo_count(const int32_t *cols, int64_t S, int64_t N, int32_t *cnt, int64_t *st) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S) return;
-  const int32_t c = cols[s];
+// Where the slots' rows and columns come from. An item is what is counted and
+// scattered: width() slots of one column.
+struct SlotList {  // any list: slot s has row rows[s] and column cols[s]
+  const int32_t *rows, *cols;
+  __device__ __forceinline__ int width() const { return 1; }
+  __device__ __forceinline__ int32_t col(int64_t item) const { return cols[item]; }
+  __device__ __forceinline__ int32_t slot(int64_t item) const { return (int32_t)item; }
+  __device__ __forceinline__ int32_t row(int32_t slot) const { return rows[slot]; }
+  // slot q of a column's list whose items' first slots are scattered
+  __device__ __forceinline__ int32_t listed(const int32_t *perm, int q) const { return perm[q]; }
+};
+
+// Element blocks: slot D^2 t + D i + j has row dofs[t][i] and column dofs[t][j]; an
+// item is column j of element t, its D slots D apart. A tenth of the atomics of a
+// list of 10 x 10 blocks and no row and column arrays: at 99,900 tets 8 + 15 us
+// for count and scatter, where the lists took 44 (k_coo_rowcol) + 166 + 216, and
+// k_coo_fill 32 instead of 48.
+template <int D_>
+struct BlockList {
+  const int32_t *dofs;  // [n_elements][D]
+  int d;
+  __device__ __forceinline__ int D() const { return D_ ? D_ : d; }
+  __device__ __forceinline__ int width() const { return D(); }
+  __device__ __forceinline__ int32_t col(int64_t item) const { return dofs[item]; }
+  __device__ __forceinline__ int32_t slot(int64_t item) const {
+    return (int32_t)(item / D() * (D() * (int64_t)D()) + item % D());
+  }
+  __device__ __forceinline__ int32_t row(int32_t slot) const {
+    const int32_t col_of = slot / D();  // D t + i
+    return dofs[col_of];
+  }
+  __device__ __forceinline__ int32_t listed(const int32_t *perm, int q) const {
+    return perm[q / D() * D()] + q % D() * D();
+  }
+};
+
+template <typename List>
+__global__ void k_coo_count(List list, int64_t items, int64_t N, int32_t *cnt, int64_t *st) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= items) return;
+  const int32_t c = list.col(k);
   if (c < 0 || c >= N) {
-    flag(st, EMG_ST_INDEX, s);
+    flag(st, EMG_ST_INDEX, list.slot(k));
     return;
   }
-  atomicAdd(&cnt[c], 1);
+  atomicAdd(&cnt[c], list.width());
 }
 
-__global__ void k_coo_scatter(const int32_t *cols, int64_t S, int64_t N, const int32_t *col_off, int32_t *cursor,
+// each item's first slot to the start of its part of the column's list
+template <typename List>
+__global__ void k_coo_scatter(List list, int64_t items, int64_t N, const int32_t *col_off, int32_t *cursor,
                               int32_t *perm) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S) return;
-  const int32_t c = cols[s];
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= items) return;
+  const int32_t c = list.col(k);
   if (c < 0 || c >= N) return;
-  perm[col_off[c] + atomicAdd(&cursor[c], 1)] = (int32_t)s;
+  perm[col_off[c] + atomicAdd(&cursor[c], list.width())] = list.slot(k);
 }
 
 // Sort each column's slots by (row, slot) and count its distinct rows: a warp per
@@ -40,17 +81,19 @@ __global__ void k_coo_scatter(const int32_t *cols, int64_t S, int64_t N, const i
 // of the slots' rows.
 constexpr int SORT_WARPS = 8;
 
-__device__ __forceinline__ uint64_t coo_key(const int32_t *rows, int32_t slot) {
-  return ((uint64_t)(uint32_t)rows[slot] << 32) | (uint32_t)slot;
+template <typename List>
+__device__ __forceinline__ uint64_t coo_key(const List &list, int32_t slot) {
+  return ((uint64_t)(uint32_t)list.row(slot) << 32) | (uint32_t)slot;
 }
 
 // sorts the column's n <= 32 K slots perm[0..n); returns its distinct rows
-template <int K>
-__device__ __forceinline__ int32_t sort_column(const int32_t *rows, int64_t N, int32_t *perm, int n, int64_t *st) {
+template <int K, typename List>
+__device__ __forceinline__ int32_t sort_column(const List &list, int64_t N, int32_t *perm, int n, int64_t *st) {
   const int lane = threadIdx.x & 31;
   uint64_t k[K];
 #pragma unroll
-  for (int r = 0; r < K; ++r) k[r] = r * 32 + lane < n ? coo_key(rows, perm[r * 32 + lane]) : ~0ull;
+  for (int r = 0; r < K; ++r) k[r] = r * 32 + lane < n ? coo_key(list, list.listed(perm, r * 32 + lane)) : ~0ull;
+  __syncwarp();  // every lane has read the list before any writes it
   warp_sort<K>(k);
   int32_t distinct = 0;
 #pragma unroll
@@ -74,8 +117,12 @@ __device__ __forceinline__ int32_t sort_column(const int32_t *rows, int64_t N, i
 // the same for a column of any length, in global memory: a bitonic network
 // whose comparators all put the smaller key first, so that those past the end
 // of the column can be left out
-__device__ int32_t sort_long_column(const int32_t *rows, int64_t N, int32_t *perm, int64_t n, int64_t *st) {
-  const int lane = threadIdx.x & 31;
+template <typename List>
+__device__ int32_t sort_long_column(const List &list, int64_t N, int32_t *perm, int64_t n, int64_t *st) {
+  const int lane = threadIdx.x & 31, width = list.width();
+  for (int64_t q = (int64_t)lane * width; width > 1 && q < n; q += 32 * (int64_t)width)  // an item's slots, in its part
+    for (int i = 1; i < width; ++i) perm[q + i] = perm[q] + i * width;
+  __syncwarp();
   for (int64_t size = 2; (size >> 1) < n; size <<= 1)
     for (int64_t j = size >> 1; j > 0; j >>= 1) {
       const bool flip = j == (size >> 1);
@@ -84,7 +131,7 @@ __device__ int32_t sort_long_column(const int32_t *rows, int64_t N, int32_t *per
         const int64_t i = block + at, o = flip ? block + 2 * j - 1 - at : i + j;
         if (o < n) {
           const int32_t a = perm[i], b = perm[o];
-          if (coo_key(rows, a) > coo_key(rows, b)) {
+          if (coo_key(list, a) > coo_key(list, b)) {
             perm[i] = b;
             perm[o] = a;
           }
@@ -94,35 +141,37 @@ __device__ int32_t sort_long_column(const int32_t *rows, int64_t N, int32_t *per
     }
   int32_t distinct = 0;
   for (int64_t i = lane; i < n; i += 32) {
-    const int32_t r = rows[perm[i]];
+    const int32_t r = list.row(perm[i]);
     if (r < 0 || r >= N) flag(st, EMG_ST_INDEX, perm[i]);
-    distinct += i == 0 || r != rows[perm[i - 1]] ? 1 : 0;
+    distinct += i == 0 || r != list.row(perm[i - 1]) ? 1 : 0;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) distinct += __shfl_xor_sync(0xffffffffu, distinct, o);
   return distinct;
 }
 
+template <typename List>
 __global__ void __launch_bounds__(SORT_WARPS * 32)
-    k_coo_sort_count(const int32_t *rows, const int32_t *col_off, int64_t N, int32_t *perm, int32_t *col_nnz,
+    k_coo_sort_count(List list, const int32_t *col_off, int64_t N, int32_t *perm, int32_t *col_nnz,
                      int64_t *st) {
   const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
   if (c >= N) return;
   const int32_t b = col_off[c], n = col_off[c + 1] - b;
   int32_t distinct;
-  if (n <= 32) distinct = sort_column<1>(rows, N, perm + b, n, st);
-  else if (n <= 64) distinct = sort_column<2>(rows, N, perm + b, n, st);
-  else if (n <= 128) distinct = sort_column<4>(rows, N, perm + b, n, st);
-  else if (n <= 256) distinct = sort_column<8>(rows, N, perm + b, n, st);
-  else if (n <= 512) distinct = sort_column<16>(rows, N, perm + b, n, st);
-  else distinct = sort_long_column(rows, N, perm + b, n, st);
+  if (n <= 32) distinct = sort_column<1>(list, N, perm + b, n, st);
+  else if (n <= 64) distinct = sort_column<2>(list, N, perm + b, n, st);
+  else if (n <= 128) distinct = sort_column<4>(list, N, perm + b, n, st);
+  else if (n <= 256) distinct = sort_column<8>(list, N, perm + b, n, st);
+  else if (n <= 512) distinct = sort_column<16>(list, N, perm + b, n, st);
+  else distinct = sort_long_column(list, N, perm + b, n, st);
   if ((threadIdx.x & 31) == 0) col_nnz[c] = distinct;
 }
 
 // indices (distinct rows) and, per entry, the first of its sorted slots: a warp
 // per column
+template <typename List>
 __global__ void __launch_bounds__(SORT_WARPS * 32)
-    k_coo_fill(const int32_t *rows, const int32_t *col_off, int64_t N, const int32_t *perm, const int32_t *indptr,
+    k_coo_fill(List list, const int32_t *col_off, int64_t N, const int32_t *perm, const int32_t *indptr,
                int32_t *indices, int32_t *run) {
   const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
   if (c >= N) return;
@@ -131,7 +180,7 @@ __global__ void __launch_bounds__(SORT_WARPS * 32)
   int32_t q = indptr[c], last = -1;
   for (int32_t i0 = b; i0 < e; i0 += 32) {
     const int32_t i = i0 + lane;
-    const int32_t r = i < e ? rows[perm[i]] : -1;
+    const int32_t r = i < e ? list.row(perm[i]) : -1;
     int32_t before = __shfl_up_sync(0xffffffffu, r, 1);
     if (lane == 0) before = last;
     const bool first = i < e && (i == b || r != before);
@@ -252,6 +301,53 @@ CooWs coo_ws(void *d_ws, int64_t N) {
   return r;
 }
 
+template <typename List>
+int coo_build(const List &list, int64_t items, emg_coo_map *m, int32_t *d_perm, void *d_ws, int32_t *d_indptr,
+              int64_t *d_status, cudaStream_t s) {
+  CooWs w = coo_ws(d_ws, m->N);
+  int rc;
+  if ((rc = status_reset(d_status, s))) return rc;
+  CUDA_TRY(cudaMemsetAsync(w.cnt, 0, (size_t)(m->N + 1) * 4, s));
+  CUDA_TRY(cudaMemsetAsync(w.cursor, 0, (size_t)(m->N + 1) * 4, s));
+  if (items > 0) {
+    k_coo_count<<<grid_for(items, 256), 256, 0, s>>>(list, items, m->N, w.cnt, d_status);
+    if ((rc = launch_check("k_coo_count"))) return rc;
+  }
+  if ((rc = scan_i32(w.cnt, m->N, w.col_off, w.bsum, d_status, s))) return rc;
+  if (items > 0) {
+    k_coo_scatter<<<grid_for(items, 256), 256, 0, s>>>(list, items, m->N, w.col_off, w.cursor, d_perm);
+    if ((rc = launch_check("k_coo_scatter"))) return rc;
+  }
+  if (m->N > 0) {
+    k_coo_sort_count<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm, w.col_nnz,
+                                                                            d_status);
+    if ((rc = launch_check("k_coo_sort_count"))) return rc;
+  }
+  if ((rc = scan_i32(w.col_nnz, m->N, d_indptr, w.bsum, d_status, s))) return rc;
+  int32_t nnz = 0;
+  int64_t h_st[2] = {0, 0};
+  CUDA_TRY(cudaMemcpyAsync(&nnz, d_indptr + m->N, 4, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaMemcpyAsync(h_st, d_status, 16, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaStreamSynchronize(s));
+  if (h_st[0]) return fail(EMG_EMESH, "COO pattern: index out of range at slot %lld", (long long)h_st[1]);
+  m->nnz = nnz;
+  return EMG_OK;
+}
+
+template <typename List>
+int coo_finish(const List &list, const emg_coo_map *m, const int32_t *d_perm, void *d_ws, const int32_t *d_indptr,
+               int32_t *d_indices, int32_t *d_run, cudaStream_t s) {
+  CooWs w = coo_ws(d_ws, m->N);
+  if (m->N > 0) {
+    k_coo_fill<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm, d_indptr,
+                                                                      d_indices, d_run);
+    const int rc = launch_check("k_coo_fill");
+    if (rc) return rc;
+  }
+  k_coo_run_end<<<1, 32, 0, s>>>(d_run, m->nnz, m->S, d_run);
+  return launch_check("k_coo_run_end");
+}
+
 }  // namespace
 }  // namespace emg
 
@@ -287,49 +383,34 @@ int emg_coo_build(emg_coo_map *m, const int32_t *d_rows, const int32_t *d_cols, 
                   int32_t *d_indptr, int64_t *d_status, emg_stream_t stream) {
   if (!m || !d_perm || !d_ws || !d_indptr || !d_status || (m->S > 0 && (!d_rows || !d_cols)))
     return fail(EMG_EINVAL, "null pointer");
-  cudaStream_t s = S(stream);
-  CooWs w = coo_ws(d_ws, m->N);
-  int rc;
-  if ((rc = status_reset(d_status, s))) return rc;
-  CUDA_TRY(cudaMemsetAsync(w.cnt, 0, (size_t)(m->N + 1) * 4, s));
-  CUDA_TRY(cudaMemsetAsync(w.cursor, 0, (size_t)(m->N + 1) * 4, s));
-  if (m->S > 0) {
-    k_coo_count<<<grid_for(m->S, 256), 256, 0, s>>>(d_cols, m->S, m->N, w.cnt, d_status);
-    if ((rc = launch_check("k_coo_count"))) return rc;
-  }
-  if ((rc = scan_i32(w.cnt, m->N, w.col_off, w.bsum, d_status, s))) return rc;
-  if (m->S > 0) {
-    k_coo_scatter<<<grid_for(m->S, 256), 256, 0, s>>>(d_cols, m->S, m->N, w.col_off, w.cursor, d_perm);
-    if ((rc = launch_check("k_coo_scatter"))) return rc;
-  }
-  if (m->N > 0) {
-    k_coo_sort_count<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(d_rows, w.col_off, m->N, d_perm, w.col_nnz, d_status);
-    if ((rc = launch_check("k_coo_sort_count"))) return rc;
-  }
-  if ((rc = scan_i32(w.col_nnz, m->N, d_indptr, w.bsum, d_status, s))) return rc;
-  int32_t nnz = 0;
-  int64_t h_st[2] = {0, 0};
-  CUDA_TRY(cudaMemcpyAsync(&nnz, d_indptr + m->N, 4, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(h_st, d_status, 16, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaStreamSynchronize(s));
-  if (h_st[0]) return fail(EMG_EMESH, "COO pattern: index out of range at slot %lld", (long long)h_st[1]);
-  m->nnz = nnz;
-  return EMG_OK;
+  return coo_build(SlotList{d_rows, d_cols}, m->S, m, d_perm, d_ws, d_indptr, d_status, S(stream));
 }
 
 int emg_coo_finish(const emg_coo_map *m, const int32_t *d_rows, const int32_t *d_perm, void *d_ws,
                    const int32_t *d_indptr, int32_t *d_indices, int32_t *d_run, emg_stream_t stream) {
   if (!m || !d_perm || !d_ws || !d_indptr || !d_run) return fail(EMG_EINVAL, "null pointer");
   if (m->nnz > 0 && (!d_indices || !d_rows)) return fail(EMG_EINVAL, "null pointer");
-  cudaStream_t s = S(stream);
-  CooWs w = coo_ws(d_ws, m->N);
-  if (m->N > 0) {
-    k_coo_fill<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(d_rows, w.col_off, m->N, d_perm, d_indptr, d_indices, d_run);
-    const int rc = launch_check("k_coo_fill");
-    if (rc) return rc;
-  }
-  k_coo_run_end<<<1, 32, 0, s>>>(d_run, m->nnz, m->S, d_run);
-  return launch_check("k_coo_run_end");
+  return coo_finish(SlotList{d_rows, nullptr}, m, d_perm, d_ws, d_indptr, d_indices, d_run, S(stream));
+}
+
+int emg_coo_build_blocks(emg_coo_map *m, const int32_t *d_dofs, int dofs_per_tet, int32_t *d_perm, void *d_ws,
+                         int32_t *d_indptr, int64_t *d_status, emg_stream_t stream) {
+  if (!m || !d_perm || !d_ws || !d_indptr || !d_status || (m->S > 0 && !d_dofs))
+    return fail(EMG_EINVAL, "null pointer");
+  const int64_t D = dofs_per_tet;
+  if (D <= 0 || m->S % (D * D)) return fail(EMG_EINVAL, "slot count is not a multiple of the block size");
+  if (D == 10) return coo_build(BlockList<10>{d_dofs, 10}, m->S / 10, m, d_perm, d_ws, d_indptr, d_status, S(stream));
+  return coo_build(BlockList<0>{d_dofs, dofs_per_tet}, m->S / D, m, d_perm, d_ws, d_indptr, d_status, S(stream));
+}
+
+int emg_coo_finish_blocks(const emg_coo_map *m, const int32_t *d_dofs, int dofs_per_tet, const int32_t *d_perm,
+                          void *d_ws, const int32_t *d_indptr, int32_t *d_indices, int32_t *d_run,
+                          emg_stream_t stream) {
+  if (!m || !d_perm || !d_ws || !d_indptr || !d_run || dofs_per_tet <= 0) return fail(EMG_EINVAL, "null pointer");
+  if (m->nnz > 0 && (!d_indices || !d_dofs)) return fail(EMG_EINVAL, "null pointer");
+  if (dofs_per_tet == 10)
+    return coo_finish(BlockList<10>{d_dofs, 10}, m, d_perm, d_ws, d_indptr, d_indices, d_run, S(stream));
+  return coo_finish(BlockList<0>{d_dofs, dofs_per_tet}, m, d_perm, d_ws, d_indptr, d_indices, d_run, S(stream));
 }
 
 int emg_coo_gather(const emg_coo_map *m, const int32_t *d_perm, const int32_t *d_run, int is_complex, int block_dofs,

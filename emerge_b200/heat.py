@@ -113,32 +113,35 @@ class GpuCOOMapping:
     them."""
 
     def __init__(self, d_rows: torch.Tensor, d_cols: torch.Tensor, N: int, device=None):
-        dev = d_rows.device
-        self.device = dev
-        self.N = int(N)
         S = int(d_rows.numel())
         if d_cols.numel() != S:
             raise ValueError("rows and cols differ in length")
-        self.block_dofs = 0  # 10 when the slots are 10x10 blocks per tet (from_tet_to_field)
+        rows = d_rows.to(torch.int32).contiguous()
+        cols = d_cols.to(torch.int32).contiguous()
+        lib = L.lib()
+        self._setup(d_rows.device, S, N, 0, lambda *a: lib.emg_coo_build(a[0], L.ptr(rows), L.ptr(cols), *a[1:]),
+                    lambda *a: lib.emg_coo_finish(a[0], L.ptr(rows), *a[1:]))
+
+    def _setup(self, dev, S: int, N: int, block_dofs: int, build, finish):
+        """The pattern and the slots' order from the slots that `build` and `finish` are given."""
+        self.device = dev
+        self.N = int(N)
+        self.block_dofs = block_dofs  # D when the slots are D x D blocks per tet (from_tet_to_field)
         m = L.CooMap()
         L.check(L.lib().emg_coo_init(S, self.N, L.ctypes.byref(m)))
         self.desc = m
         self.S = S
-        self._rows = d_rows.to(torch.int32).contiguous()
-        cols = d_cols.to(torch.int32).contiguous()
         self.d_perm = torch.empty(m.perm_bytes // 4, dtype=torch.int32, device=dev)
         ws = torch.empty(max(m.workspace_bytes, 1), dtype=torch.uint8, device=dev)
         self.d_indptr = torch.empty(self.N + 1, dtype=torch.int32, device=dev)
         status = torch.zeros(2, dtype=torch.int64, device=dev)
         st = L.stream_handle(dev)
-        L.check(L.lib().emg_coo_build(L.ctypes.byref(m), L.ptr(self._rows), L.ptr(cols), L.ptr(self.d_perm),
-                                      L.ptr(ws), L.ptr(self.d_indptr), L.ptr(status), st))
+        L.check(build(L.ctypes.byref(m), L.ptr(self.d_perm), L.ptr(ws), L.ptr(self.d_indptr), L.ptr(status), st))
         self.nnz = int(m.nnz)
         self.d_indices = torch.empty(max(self.nnz, 1), dtype=torch.int32, device=dev)
         self.d_run = torch.empty(self.nnz + 1, dtype=torch.int32, device=dev)
-        L.check(L.lib().emg_coo_finish(L.ctypes.byref(m), L.ptr(self._rows), L.ptr(self.d_perm), L.ptr(ws),
-                                       L.ptr(self.d_indptr), L.ptr(self.d_indices), L.ptr(self.d_run), st))
-        self._rows = None  # the rows live on in d_indices
+        L.check(finish(L.ctypes.byref(m), L.ptr(self.d_perm), L.ptr(ws), L.ptr(self.d_indptr), L.ptr(self.d_indices),
+                       L.ptr(self.d_run), st))
         self._indptr = self._indices = None
 
     @staticmethod
@@ -169,14 +172,11 @@ class GpuCOOMapping:
         D, nT = t2f.shape
         if t2f.size and (t2f.min() < 0 or t2f.max() >= N):
             raise IndexError("tet_to_field entry outside [0, N)")
-        d_t2f = _to_dev(t2f, torch.int32, dev)
-        S = D * D * nT
-        rows = torch.empty(max(S, 1), dtype=torch.int32, device=dev)
-        cols = torch.empty(max(S, 1), dtype=torch.int32, device=dev)
-        L.check(L.lib().emg_coo_rowcol(L.ptr(d_t2f), int(D), int(nT), L.ptr(rows), L.ptr(cols),
-                                       L.stream_handle(dev)))
-        cm = GpuCOOMapping(rows[:S], cols[:S], N)
-        cm.block_dofs = int(D)
+        dofs = _to_dev(t2f, torch.int32, dev).t().contiguous()  # a tet's DoFs side by side
+        lib = L.lib()
+        cm = GpuCOOMapping.__new__(GpuCOOMapping)
+        cm._setup(dev, D * D * nT, N, int(D), lambda *a: lib.emg_coo_build_blocks(a[0], L.ptr(dofs), int(D), *a[1:]),
+                  lambda *a: lib.emg_coo_finish_blocks(a[0], L.ptr(dofs), int(D), *a[1:]))
         return cm
 
     @property

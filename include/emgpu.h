@@ -519,6 +519,15 @@ int emg_coo_build(emg_coo_map *map, const int32_t *d_rows, const int32_t *d_cols
                   int32_t *d_indptr, int64_t *d_status, emg_stream_t stream);
 int emg_coo_finish(const emg_coo_map *map, const int32_t *d_rows, const int32_t *d_perm, void *d_workspace,
                    const int32_t *d_indptr, int32_t *d_indices, int32_t *d_run, emg_stream_t stream);
+/* The same for the D x D blocks of elements, slot D^2 t + D i + j with row
+ * d_dofs[t][i] and column d_dofs[t][j] (S = D^2 times the elements; d_dofs int32
+ * [n_elements][D], needed until emg_coo_finish_blocks): the mapping that
+ * emg_coo_rowcol's lists give, without the lists. */
+int emg_coo_build_blocks(emg_coo_map *map, const int32_t *d_dofs, int dofs_per_tet, int32_t *d_perm, void *d_workspace,
+                         int32_t *d_indptr, int64_t *d_status, emg_stream_t stream);
+int emg_coo_finish_blocks(const emg_coo_map *map, const int32_t *d_dofs, int dofs_per_tet, const int32_t *d_perm,
+                          void *d_workspace, const int32_t *d_indptr, int32_t *d_indices, int32_t *d_run,
+                          emg_stream_t stream);
 /* CSC values (f64, or complex128 when is_complex) from slot values:
  * block_dofs 0 reads slot s at d_values[s]; block_dofs 10 reads values stored
  * as transposed 10x10 blocks (EMG_LAYOUT_COO_T) of slots 100 t + 10 i + j. */
