@@ -673,11 +673,11 @@ def run_sweep(args, rank, world, local_rank):
                        "tets": f.ntets, "nnz": nnz, "freqs": nf,
                        "band_hz": [8e9, 12e9], "batch": nb, "port_tris": int(sum(r.n_btris for r in ports)),
                        "K_M_form": "fp64", "setup_s": setup_s, "l2": l2.text(),
-                       "step": f"all {nf} frequencies, {n_launch} form launches + {2 * nf} port-term launches"},
+                       "step": f"all {nf} frequencies, {n_launch} form launches + {2 * n_launch} port-term launches"},
             "tet_freqs_per_s": world * f.ntets * nf / (ms * 1e-3),
             "roofline": {"bound": "hbm", "kernel": "k_form_sweep", "achieved": ach, "peak": hbm, "unit": "GB/s",
                          "frac": ach / hbm, "alg_bytes_per_step": bytes_sweep, "traffic": None},
-            "clocks": sampler.summary(), "gpu_launches": args.steps * (n_launch + 2 * nf)}, wl
+            "clocks": sampler.summary(), "gpu_launches": args.steps * 3 * n_launch}, wl
 
 
 def run_pml(args, rank, world, local_rank):

@@ -1082,8 +1082,8 @@ __device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsi
 // A mesh that leaves most of the GPU idle: its tets are gone through by several
 // CTAs, blockIdx.y of n_parts, each of which forms the geometry and moments again
 // but only some of the block rows (row i has 10 - i blocks). The time of such a
-// launch is that of one tet: 4,950 tets mixed 20.5 -> 12.3 us and FP64 28.7 -> 20.5
-// in five parts, 12,960 mixed 21.5 -> 14.4 in five and FP64 28.7 -> 26.6 in two.
+// launch is that of one tet: 4,950 tets FP64 22.6 -> 18.5 us and mixed 12.3 -> 10.2
+// in five parts, 12,960 mixed 13.3 -> 12.3 in five and FP64 22.6 either way in two.
 // More parts than fit at once would put the repeated part into a second wave.
 constexpr unsigned ALL_ROWS = 0x3ffu;
 __device__ __forceinline__ unsigned part_rows(int part, int n_parts) {
