@@ -46,8 +46,9 @@ enum { FORM_REF64 = 0, FORM_REF32 = 1, FORM_EXACT = 2 };
 // -> 1,110 us (EXACT 726 -> 660), full at 414,720 1,856 -> 555 (1,276 -> 361).
 // Bound: FP64 latency at eight warps per SM (254 registers).
 // Full tensors go through their symmetric halves first (all there is to a
-// reciprocal material); a warp that has any other adds the antisymmetric halves'
-// part in a second pass (both halves in one pass kept 4.9 KB spilled: 1,607 us).
+// reciprocal material); where a warp has any other, those tets add the
+// antisymmetric halves' part in a second pass (both halves in one pass kept 4.9 KB
+// spilled: 1,607 us).
 enum { KIND_PAIR = 3, KIND_PAIR_FULL = 4, KIND_PAIR_ANTI = 5 };
 __host__ __device__ constexpr int tensor_kind(int form, int kind) {
   return form == FORM_REF32 || kind == EMG_MAT_ISO ? kind : (kind == EMG_MAT_DIAG ? KIND_PAIR : KIND_PAIR_FULL);
@@ -1037,6 +1038,9 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
                      t[5].re == t[7].re && t[5].im == t[7].im;
             };
             asym = KIND == EMG_MAT_FULL && !(symmetric(eps) && symmetric(mu3));
+            // a reciprocal tet keeps the first pass's values whatever its neighbours are:
+            // the inverse of its mu may be symmetric only up to rounding
+            if (TK == KIND_PAIR_ANTI) active = asym;
             double e[9], u[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
