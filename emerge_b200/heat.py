@@ -234,39 +234,65 @@ class GpuCOOMapping:
         return csc_matrix((vals, self.indices, self.indptr), shape=(self.N, self.N))
 
 
-class _HeatMesh:
-    """Nodes, tets and the COO mapping of one field, kept on the device and
-    reused by the stiffness and mass calls of that field."""
+def _bits(a: np.ndarray) -> torch.Tensor:
+    """A host array's values bit for bit, as a torch tensor (its copies and
+    comparisons use all host threads)."""
+    b = np.ascontiguousarray(a).reshape(-1)
+    return torch.from_numpy(b.view(np.int64 if b.nbytes % 8 == 0 else np.uint8))
 
-    def __init__(self, field, device):
-        m = field.mesh
-        t2f = np.asarray(field.tet_to_field)
+
+class _HeatTopology:
+    """Tets and the COO mapping of one field, kept on the device with host
+    copies of the arrays that they were made from."""
+
+    def __init__(self, field, tets: np.ndarray, t2f: np.ndarray, n_nodes: int, device):
         if t2f.ndim != 2 or t2f.shape[0] != 10:
             raise ValueError("tet_to_field must be [10, n_tets]")
-        self.n_nodes, self.n_tets = int(m.n_nodes), int(np.asarray(m.tets).shape[1])
+        self.n_tets = int(tets.shape[1])
         if t2f.shape[1] != self.n_tets:
             raise ValueError("tet_to_field and mesh.tets differ in tet count")
-        self.nodes = _to_dev(np.asarray(m.nodes, dtype=np.float64), torch.float64, device)
-        t = np.asarray(m.tets)
-        if t.size and (t.min() < 0 or t.max() >= self.n_nodes):  # before narrowing to int32
+        if tets.size and (tets.min() < 0 or tets.max() >= n_nodes):  # before narrowing to int32
             raise IndexError("tet node index outside [0, n_nodes)")
-        self.tets = _to_dev(t, torch.int32, device)
+        self.field = field
+        self.sizes = (n_nodes, int(field.n_field), device)
+        self.made_from = [(a.dtype, a.shape, _bits(a).clone()) for a in (tets, t2f)]
+        self.tets = _to_dev(tets, torch.int32, device)
         self.cmap = GpuCOOMapping.from_tet_to_field(t2f, int(field.n_field), device)
-        self.key = (id(m.nodes), id(m.tets), id(field.tet_to_field), int(field.n_field))
+
+    def fits(self, field, tets: np.ndarray, t2f: np.ndarray, n_nodes: int, device) -> bool:
+        """Whether it was made of this field as the field's arrays are now. They
+        are compared value by value: a partitioned field may be renumbered in
+        place, and an array's id is given to the next one once it is gone."""
+        if self.field is not field or self.sizes != (n_nodes, int(field.n_field), device):
+            return False
+        return all(a.dtype == dtype and a.shape == shape and torch.equal(_bits(a), bits)
+                   for a, (dtype, shape, bits) in zip((tets, t2f), self.made_from))
 
 
-_CACHE: dict = {}
+class _HeatMesh:
+    """Nodes, tets and the COO mapping for one call."""
+
+    def __init__(self, topology: _HeatTopology, nodes: torch.Tensor, n_nodes: int):
+        self.n_nodes, self.n_tets, self.nodes = n_nodes, topology.n_tets, nodes
+        self.tets, self.cmap = topology.tets, topology.cmap
+
+
+_KEPT: _HeatTopology | None = None
 
 
 def _heat_mesh(field, device) -> _HeatMesh:
-    dev = _device(device)
-    h = _CACHE.get(id(field))
-    key = (id(field.mesh.nodes), id(field.mesh.tets), id(field.tet_to_field), int(field.n_field))
-    if h is None or h[0] is not field or h[1].key != key or h[1].nodes.device != dev:
-        _CACHE.clear()  # one field resident at a time
-        h = (field, _HeatMesh(field, dev))
-        _CACHE[id(field)] = h
-    return h[1]
+    """The coordinates are uploaded on every call; tets and mapping are kept for
+    the stiffness and mass calls of a field."""
+    global _KEPT
+    dev, m = _device(device), field.mesh
+    if dev.index is None:
+        dev = torch.device("cuda", torch.cuda.current_device())
+    tets, t2f, n_nodes = np.asarray(m.tets), np.asarray(field.tet_to_field), int(m.n_nodes)
+    kept = _KEPT
+    if kept is None or not kept.fits(field, tets, t2f, n_nodes, dev):
+        kept = _KEPT = None  # one field resident at a time
+        kept = _KEPT = _HeatTopology(field, tets, t2f, n_nodes, dev)
+    return _HeatMesh(kept, _to_dev(np.asarray(m.nodes, dtype=np.float64), torch.float64, dev), n_nodes)
 
 
 def _element(field, coef: np.ndarray, kind: int, precision: str, device) -> tuple[CooValues, GpuCOOMapping]:
