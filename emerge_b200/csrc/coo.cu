@@ -176,10 +176,10 @@ __global__ void __launch_bounds__(SORT_WARPS * 32)
   const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
   if (c >= N) return;
   const int lane = threadIdx.x & 31;
-  const int32_t b = col_off[c], e = col_off[c + 1];
+  const int64_t b = col_off[c], e = col_off[c + 1];
   int32_t q = indptr[c], last = -1;
-  for (int32_t i0 = b; i0 < e; i0 += 32) {
-    const int32_t i = i0 + lane;
+  for (int64_t i0 = b; i0 < e; i0 += 32) {  // i0 passes e, which may be nearly the last int32
+    const int64_t i = i0 + lane;
     const int32_t r = i < e ? list.row(perm[i]) : -1;
     int32_t before = __shfl_up_sync(0xffffffffu, r, 1);
     if (lane == 0) before = last;
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(SORT_WARPS * 32)
     if (first) {
       const int32_t at = q + __popc(m & ((1u << lane) - 1u));
       indices[at] = r;
-      run[at] = i;
+      run[at] = (int32_t)i;
     }
     q += __popc(m);
     last = __shfl_sync(0xffffffffu, r, 31);
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256, 8) k_coo_gather_f8(const int32_t *perm, c
     }
     double s = 0.0;
     int32_t i = b;
-    for (; i + 4 <= e; i += 4) {  // four loads in flight, summed in slot order
+    for (; e - i >= 4; i += 4) {  // four loads in flight, summed in slot order
       const int32_t p0 = perm[i], p1 = perm[i + 1], p2 = perm[i + 2], p3 = perm[i + 3];
       const double v0 = vals[value_index<D>(p0)], v1 = vals[value_index<D>(p1)];
       const double v2 = vals[value_index<D>(p2)], v3 = vals[value_index<D>(p3)];
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256, 8) k_coo_gather_f8(const int32_t *perm, c
       s += v2;
       s += v3;
     }
-    if (i + 2 <= e) {
+    if (e - i >= 2) {
       const int32_t p0 = perm[i], p1 = perm[i + 1];
       const double v0 = vals[value_index<D>(p0)], v1 = vals[value_index<D>(p1)];
       s += v0;

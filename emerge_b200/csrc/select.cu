@@ -31,8 +31,8 @@ __global__ void __launch_bounds__(256)
   const int l = threadIdx.x % SEL_LANES;
   int32_t c = 0;
   if (j < N && keep[j]) {
-    const int32_t e = indptr[j + 1];
-    for (int32_t p = indptr[j] + l; p < e; p += SEL_LANES) {
+    const int64_t e = indptr[j + 1];
+    for (int64_t p = (int64_t)indptr[j] + l; p < e; p += SEL_LANES) {  // p passes e, which may be the last int32
       const int32_t r = indices[p];
       if (r < 0 || r >= N) {
         flag(st, EMG_ST_INDEX, p);
@@ -60,10 +60,11 @@ __global__ void __launch_bounds__(256)
                const int32_t *indptr_sel, int32_t *indices_sel, int32_t *take) {
   const int64_t j = (int64_t)blockIdx.x * SEL_COLS + threadIdx.x / SEL_LANES;
   const int lane = threadIdx.x & 31, l = lane % SEL_LANES;
-  int32_t q = 0, p = 0, e = 0;
+  int32_t q = 0;
+  int64_t p = 0, e = 0;
   if (j < N && keep[j]) {
     q = indptr_sel[newid[j]];
-    p = indptr[j] + l;
+    p = (int64_t)indptr[j] + l;
     e = indptr[j + 1];
   }
   while (__any_sync(0xffffffffu, p - l < e)) {
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(256)
     if (in) {
       const int32_t at = q + __popc(m & ((1u << l) - 1u));
       indices_sel[at] = id;
-      take[at] = p;
+      take[at] = (int32_t)p;
     }
     q += __popc(m);
     p += SEL_LANES;
