@@ -519,24 +519,35 @@ __global__ void __launch_bounds__(CC_WARPS * 32)
       const uint32_t pos = item_byte(own, 5 + r), same = pos * 0x01010101u;
       // bytes of an item: slot at 4, pos[0..9] at 5..14 (edges, then faces), ranks at 15
       const uint32_t my = r < 6 ? 0xffffff00u : 0u, mz = r < 6 ? 0x00ffffffu : 0xff000000u, mw = r < 6 ? 0u : 0x00ffffffu;
+      // the first row slot of item o that holds this row entity, -1 if none does:
+      // the first matching byte, less the five before pos
+      auto slot_in = [&](const uint4 &o) {
+        const uint32_t hy = __vcmpeq4(o.y, same) & my, hz = __vcmpeq4(o.z, same) & mz, hw = __vcmpeq4(o.w, same) & mw;
+        if (!(hy | hz | hw)) return -1;
+        return (hy ? __ffs(hy) / 8 : (hz ? 4 + __ffs(hz) / 8 : 8 + __ffs(hw) / 8)) - 1;
+      };
+      const uint32_t word = word_of(own, r);
+      const int slot = (int)item_byte(own, 4);
+      if (r == slot) words[2 * H + (k - I0)] = word;
+      // a tet that lists a row entity twice, which only inconsistent topology arrays
+      // do, counts once: more would not fit the chunk's words
+      if (slot_in(own) != r) continue;
       const int i0 = m.ptr[e], i1 = m.ptr[e + 1];
       int total = 0, rank = 0, other = k, other_r = r;
       for (int i = i0; i < i1; ++i) {
-        const uint4 o = raw[i];
-        const uint32_t hy = __vcmpeq4(o.y, same) & my, hz = __vcmpeq4(o.z, same) & mz, hw = __vcmpeq4(o.w, same) & mw;
-        if (hy | hz | hw) {
+        const int at = slot_in(raw[i]);
+        if (at >= 0) {
           ++total;
           rank += i < k ? 1 : 0;
           if (i != k) {
-            other = i;  // its row slot: the first matching byte, less the five before pos
-            other_r = (hy ? __ffs(hy) / 8 : (hz ? 4 + __ffs(hz) / 8 : 8 + __ffs(hw) / 8)) - 1;
+            other = i;
+            other_r = at;
           }
         }
       }
       const int h = (m.c0[e] - A0) / 2 + (r < 6 ? 0 : m.ne[e]) + (int)pos;
-      const uint32_t word = word_of(own, r);
-      const bool self = r == (int)item_byte(own, 4);  // the entity's pair with itself: every item has one
-      if (self) words[2 * H + (k - I0)] = word;
+      // the entity's pair with itself: every item has one
+      const bool self = (r < 6) == (slot < 6) && item_byte(own, 5 + slot) == pos;
       // two blocks stored different ways round: only with inconsistent topology arrays
       const bool differ = total == 2 && ((word_of(raw[other], other_r) ^ word) >> 31);
       if (total <= 2 && !differ) {
