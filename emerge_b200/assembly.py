@@ -62,7 +62,8 @@ def _empty(numel: int, dtype: torch.dtype, dev: torch.device, alloc=None) -> tor
 
 def _to_dev(a: np.ndarray, dtype: torch.dtype, dev: torch.device, alloc=None) -> torch.Tensor:
     if alloc is None:
-        if isinstance(a, np.ndarray) and a.ndim == 2 and a.flags.f_contiguous and not a.flags.c_contiguous:
+        if (isinstance(a, np.ndarray) and a.ndim == 2 and a.flags.f_contiguous and not a.flags.c_contiguous
+                and a.flags.writeable):
             # laid out the other way round: uploaded as it is and turned over there;
             # done before this returns, as a plain upload is, whatever stream reads it next
             t = torch.from_numpy(a.T).to(device=dev, dtype=dtype, non_blocking=False).T.contiguous()

@@ -1,5 +1,7 @@
 """Host arrays of either memory order reach the device whole before the upload
 returns, so that any stream may read them."""
+import warnings
+
 import numpy as np
 import pytest
 import torch
@@ -22,3 +24,12 @@ def test_upload_is_complete(order, host, dtype):
         done = stream.query()
     assert done
     assert t.is_contiguous() and torch.equal(t.cpu(), torch.from_numpy(np.ascontiguousarray(a)).to(dtype))
+
+
+def test_read_only_array():
+    a = np.asfortranarray(np.arange(12.0).reshape(3, 4))
+    a.setflags(write=False)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        t = _to_dev(a, torch.float64, torch.device("cuda", torch.cuda.current_device()))
+    assert torch.equal(t.cpu(), torch.from_numpy(a.copy()))
