@@ -1083,12 +1083,17 @@ __device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsi
     if (asym) element_pass<FORM, KIND, LAYOUT, KIND_PAIR_ANTI>(a, ia0, rows, stage_raw);
 }
 
-// A mesh that leaves most of the GPU idle: its tets are gone through by several
-// CTAs, blockIdx.y of n_parts, each of which forms the geometry and moments again
-// but only some of the block rows (row i has 10 - i blocks). The time of such a
-// launch is that of one tet: 4,950 tets FP64 22.6 -> 18.5 us and mixed 12.3 -> 10.2
-// in five parts, 12,960 mixed 13.3 -> 12.3 in five and FP64 22.6 either way in two.
-// More parts than fit at once would put the repeated part into a second wave.
+// A mesh that leaves SMs idle: its tets are gone through by several CTAs,
+// blockIdx.y of n_parts, each of which forms the geometry and moments again but only
+// some of the block rows (row i has 10 - i blocks). The time of such a launch is that
+// of one tet. As many parts as give each CTA an SM of its own. One assembly (element
+// and gather, graph replays) on one stream, and per assembly with eight streams at
+// once, whole -> in parts: 576 tets FP64 (five parts) 23.0 -> 16.7 us and 3.6 -> 2.9;
+// 4,950 (three) FP64 27.1 -> 21.6 and 11.6 -> 13.3, mixed 16.7 -> 14.4 and 8.9 -> 8.4;
+// 8,640 (two) FP64 33.2 -> 29.1 and 19.2 -> 20.7, mixed 21.2 -> 19.7 and 14.5 -> 14.2.
+// As many parts as fit two CTAs per SM (five, three, two at 12,960 tets): FP64 22.9, 30.5
+// and 42.1 us, no faster, but 15.4, 22.5 and 31.0 with eight streams, as the repeated
+// part takes the other launches' SMs.
 constexpr unsigned ALL_ROWS = 0x3ffu;
 __device__ __forceinline__ unsigned part_rows(int part, int n_parts) {
   if (n_parts == 2) return part ? 0x3f8u : 0x007u;                                  // 27 and 28 blocks
@@ -1137,12 +1142,6 @@ __global__ void __launch_bounds__(ELEM_THREADS, elem_min_blocks<FORM, KIND>())
   element_cta<FORM, KIND, LAYOUT>(jobs[lo], (b - cta_start[lo]) * elem_tets<FORM, KIND>(), ALL_ROWS, stage_raw);
 }
 
-// CTAs that share an SM, by registers and stage
-template <int FORM, int KIND>
-constexpr int elem_ctas_per_sm() {
-  return FORM == FORM_REF32 ? (KIND == EMG_MAT_ISO ? 5 : (KIND == EMG_MAT_DIAG ? 3 : 2)) : 2;
-}
-
 template <int FORM, int KIND, int LAYOUT>
 int launch_element_t(const ElemArgs &a, cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
@@ -1163,9 +1162,9 @@ int launch_element_t(const ElemArgs &a, cudaStream_t s) {
   if (a.nA == 0) return EMG_OK;
   const int ctas = grid_for(a.nA, elem_tets<FORM, KIND>());
   int parts = 1;
-  if (LAYOUT == 2)  // the most parts that still fit the GPU at once
+  if (LAYOUT == 2)  // the most parts that still have an SM each
     for (int p : {2, 3, 5})
-      if ((int64_t)ctas * p <= persistent_ctas(elem_ctas_per_sm<FORM, KIND>())) parts = p;
+      if ((int64_t)ctas * p <= persistent_ctas(1)) parts = p;
   k_element<FORM, KIND, LAYOUT><<<dim3(ctas, parts), ELEM_THREADS, smem, s>>>(a);
   return launch_check("k_element");
 }
