@@ -150,34 +150,24 @@ __device__ int32_t sort_long_column(const List &list, int64_t N, int32_t *perm, 
   return distinct;
 }
 
+// one warp, a column of any length
 template <typename List>
-__global__ void __launch_bounds__(SORT_WARPS * 32)
-    k_coo_sort_count(List list, const int32_t *col_off, int64_t N, int32_t *perm, int32_t *col_nnz,
-                     int64_t *st) {
-  const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
-  if (c >= N) return;
-  const int32_t b = col_off[c], n = col_off[c + 1] - b;
-  int32_t distinct;
-  if (n <= 32) distinct = sort_column<1>(list, N, perm + b, n, st);
-  else if (n <= 64) distinct = sort_column<2>(list, N, perm + b, n, st);
-  else if (n <= 128) distinct = sort_column<4>(list, N, perm + b, n, st);
-  else if (n <= 256) distinct = sort_column<8>(list, N, perm + b, n, st);
-  else if (n <= 512) distinct = sort_column<16>(list, N, perm + b, n, st);
-  else distinct = sort_long_column(list, N, perm + b, n, st);
-  if ((threadIdx.x & 31) == 0) col_nnz[c] = distinct;
+__device__ int32_t sort_any_column(const List &list, int64_t N, int32_t *perm, int n, int64_t *st) {
+  if (n <= 32) return sort_column<1>(list, N, perm, n, st);
+  if (n <= 64) return sort_column<2>(list, N, perm, n, st);
+  if (n <= 128) return sort_column<4>(list, N, perm, n, st);
+  if (n <= 256) return sort_column<8>(list, N, perm, n, st);
+  if (n <= 512) return sort_column<16>(list, N, perm, n, st);
+  return sort_long_column(list, N, perm, n, st);
 }
 
 // indices (distinct rows) and, per entry, the first of its sorted slots: a warp
 // per column
 template <typename List>
-__global__ void __launch_bounds__(SORT_WARPS * 32)
-    k_coo_fill(List list, const int32_t *col_off, int64_t N, const int32_t *perm, const int32_t *indptr,
-               int32_t *indices, int32_t *run) {
-  const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
-  if (c >= N) return;
+__device__ __forceinline__ void fill_column(const List &list, int64_t b, int64_t e, int32_t q, const int32_t *perm,
+                                            int32_t *indices, int32_t *run) {
   const int lane = threadIdx.x & 31;
-  const int64_t b = col_off[c], e = col_off[c + 1];
-  int32_t q = indptr[c], last = -1;
+  int32_t last = -1;
   for (int64_t i0 = b; i0 < e; i0 += 32) {  // i0 passes e, which may be nearly the last int32
     const int64_t i = i0 + lane;
     const int32_t r = i < e ? list.row(perm[i]) : -1;
@@ -192,6 +182,104 @@ __global__ void __launch_bounds__(SORT_WARPS * 32)
     }
     q += __popc(m);
     last = __shfl_sync(0xffffffffu, r, 31);
+  }
+}
+
+template <typename List>
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+    k_coo_sort_count(List list, const int32_t *col_off, int64_t N, int32_t *perm, int32_t *col_nnz,
+                     int64_t *st) {
+  const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
+  if (c >= N) return;
+  const int32_t b = col_off[c], n = col_off[c + 1] - b;
+  const int32_t distinct = sort_any_column(list, N, perm + b, n, st);
+  if ((threadIdx.x & 31) == 0) col_nnz[c] = distinct;
+}
+
+template <typename List>
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+    k_coo_fill(List list, const int32_t *col_off, int64_t N, const int32_t *perm, const int32_t *indptr,
+               int32_t *indices, int32_t *run) {
+  const int64_t c = (int64_t)blockIdx.x * SORT_WARPS + (threadIdx.x >> 5);
+  if (c >= N) return;
+  fill_column(list, col_off[c], col_off[c + 1], indptr[c], perm, indices, run);
+}
+
+// Columns that hold few slots on average (a list of scattered entries, empty
+// columns): a lane per column, and the warp together for those of its 32 that are
+// longer than COO_LANE slots. The whole mapping of random slots, a warp per column
+// -> this: 2M columns, no slots 0.75 -> 0.18 ms, 2M slots 0.97 -> 0.24, 6M 1.17 ->
+// 0.37; 1M columns, 8M 0.77 -> 0.52, 10M 0.86 -> 0.64, 16M 1.11 -> 0.92. But 20,000
+// columns, 200,000 slots 0.152 -> 0.183: from 10 slots per column on there are longer
+// columns in every warp, and few columns leave it too few warps.
+constexpr int COO_LANE = 8;
+constexpr int COO_SHORT = 10;  // slots per column, on average
+
+// one lane, n <= COO_LANE slots
+template <typename List>
+__device__ __forceinline__ int32_t sort_short_column(const List &list, int64_t N, int32_t *perm, int n, int64_t *st) {
+  uint64_t k[COO_LANE];
+#pragma unroll
+  for (int q = 0; q < COO_LANE; ++q) k[q] = q < n ? coo_key(list, list.listed(perm, q)) : ~0ull;
+#pragma unroll
+  for (int round = 0; round < COO_LANE; ++round)
+#pragma unroll
+    for (int q = round & 1; q + 1 < COO_LANE; q += 2) {
+      const uint64_t lo = k[q] < k[q + 1] ? k[q] : k[q + 1], hi = k[q] < k[q + 1] ? k[q + 1] : k[q];
+      k[q] = lo;
+      k[q + 1] = hi;
+    }
+  int32_t distinct = 0;
+#pragma unroll
+  for (int q = 0; q < COO_LANE; ++q) {
+    if (q >= n) continue;
+    const int32_t row = (int32_t)(k[q] >> 32), slot = (int32_t)(uint32_t)k[q];
+    perm[q] = slot;
+    if (row < 0 || row >= N) flag(st, EMG_ST_INDEX, slot);
+    distinct += q == 0 || row != (int32_t)(k[q > 0 ? q - 1 : 0] >> 32) ? 1 : 0;
+  }
+  return distinct;
+}
+
+template <typename List>
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+    k_coo_sort_count_short(List list, const int32_t *col_off, int64_t N, int32_t *perm, int32_t *col_nnz,
+                           int64_t *st) {
+  const int64_t c = (int64_t)blockIdx.x * (SORT_WARPS * 32) + threadIdx.x;
+  const int32_t b = c < N ? col_off[c] : 0, n = c < N ? col_off[c + 1] - b : 0;
+  int32_t distinct = n <= COO_LANE ? sort_short_column(list, N, perm + b, n, st) : 0;
+  for (unsigned more = __ballot_sync(0xffffffffu, n > COO_LANE); more; more &= more - 1) {
+    const int src = __ffs(more) - 1;
+    const int32_t bs = __shfl_sync(0xffffffffu, b, src), ns = __shfl_sync(0xffffffffu, n, src);
+    const int32_t d = sort_any_column(list, N, perm + bs, ns, st);
+    if ((threadIdx.x & 31) == src) distinct = d;
+  }
+  if (c < N) col_nnz[c] = distinct;
+}
+
+template <typename List>
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+    k_coo_fill_short(List list, const int32_t *col_off, int64_t N, const int32_t *perm, const int32_t *indptr,
+                     int32_t *indices, int32_t *run) {
+  const int64_t c = (int64_t)blockIdx.x * (SORT_WARPS * 32) + threadIdx.x;
+  const int32_t b = c < N ? col_off[c] : 0, e = c < N ? col_off[c + 1] : 0, n = e - b;
+  int32_t q = c < N ? indptr[c] : 0;
+  for (unsigned more = __ballot_sync(0xffffffffu, n > COO_LANE); more; more &= more - 1) {
+    const int src = __ffs(more) - 1;
+    fill_column(list, __shfl_sync(0xffffffffu, b, src), __shfl_sync(0xffffffffu, e, src),
+                __shfl_sync(0xffffffffu, q, src), perm, indices, run);
+  }
+  if (n > COO_LANE) return;
+  int32_t before = -1;
+#pragma unroll
+  for (int i = 0; i < COO_LANE; ++i) {
+    if (i >= n) break;
+    const int32_t r = list.row(perm[b + i]);
+    if (i == 0 || r != before) {
+      indices[q] = r;
+      run[q++] = b + i;
+    }
+    before = r;
   }
 }
 
@@ -319,8 +407,12 @@ int coo_build(const List &list, int64_t items, emg_coo_map *m, int32_t *d_perm, 
     if ((rc = launch_check("k_coo_scatter"))) return rc;
   }
   if (m->N > 0) {
-    k_coo_sort_count<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm, w.col_nnz,
-                                                                            d_status);
+    if (m->S < COO_SHORT * m->N)
+      k_coo_sort_count_short<<<grid_for(m->N, SORT_WARPS * 32), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm,
+                                                                                         w.col_nnz, d_status);
+    else
+      k_coo_sort_count<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm, w.col_nnz,
+                                                                              d_status);
     if ((rc = launch_check("k_coo_sort_count"))) return rc;
   }
   if ((rc = scan_i32(w.col_nnz, m->N, d_indptr, w.bsum, d_status, s))) return rc;
@@ -339,8 +431,12 @@ int coo_finish(const List &list, const emg_coo_map *m, const int32_t *d_perm, vo
                int32_t *d_indices, int32_t *d_run, cudaStream_t s) {
   CooWs w = coo_ws(d_ws, m->N);
   if (m->N > 0) {
-    k_coo_fill<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm, d_indptr,
-                                                                      d_indices, d_run);
+    if (m->S < COO_SHORT * m->N)
+      k_coo_fill_short<<<grid_for(m->N, SORT_WARPS * 32), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm,
+                                                                                   d_indptr, d_indices, d_run);
+    else
+      k_coo_fill<<<grid_for(m->N, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(list, w.col_off, m->N, d_perm, d_indptr,
+                                                                        d_indices, d_run);
     const int rc = launch_check("k_coo_fill");
     if (rc) return rc;
   }
