@@ -60,10 +60,16 @@ def _empty(numel: int, dtype: torch.dtype, dev: torch.device, alloc=None) -> tor
     return torch.empty(int(numel), dtype=dtype, device=dev)
 
 
+# Values of a column-major array from which the device turns it over: f8[3, n] at n =
+# 1,000 takes 38 us turned on the host and 60 on the device, 10,000 45 / 53, 30,000
+# 95 / 81, 300,000 1,227 / 455.
+_TURN_ON_DEVICE = 65536
+
+
 def _to_dev(a: np.ndarray, dtype: torch.dtype, dev: torch.device, alloc=None) -> torch.Tensor:
     if alloc is None:
         if (isinstance(a, np.ndarray) and a.ndim == 2 and a.flags.f_contiguous and not a.flags.c_contiguous
-                and a.flags.writeable):
+                and a.flags.writeable and a.size >= _TURN_ON_DEVICE):
             # laid out the other way round: uploaded as it is and turned over there;
             # done before this returns, as a plain upload is, whatever stream reads it next
             t = torch.from_numpy(a.T).to(device=dev, dtype=dtype, non_blocking=False).T.contiguous()

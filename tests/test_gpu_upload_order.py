@@ -27,9 +27,17 @@ def test_upload_is_complete(order, host, dtype):
 
 
 def test_read_only_array():
-    a = np.asfortranarray(np.arange(12.0).reshape(3, 4))
+    a = np.asfortranarray(np.arange(120_000.0).reshape(3, -1))
     a.setflags(write=False)
     with warnings.catch_warnings():
         warnings.simplefilter("error")
         t = _to_dev(a, torch.float64, torch.device("cuda", torch.cuda.current_device()))
     assert torch.equal(t.cpu(), torch.from_numpy(a.copy()))
+
+
+@pytest.mark.parametrize("n", [1, 2, 21845, 21846])
+def test_either_side_turns_it(n):
+    """65,536 values and more are turned over on the device."""
+    a = np.asfortranarray(np.arange(3 * n).reshape(3, n))
+    t = _to_dev(a, torch.int32, torch.device("cuda", torch.cuda.current_device()))
+    assert t.is_contiguous() and torch.equal(t.cpu(), torch.from_numpy(a.copy()).to(torch.int32))
