@@ -52,10 +52,11 @@ class SolveSubmatrix:
         ids = np.asarray(solve_ids, dtype=np.int64).ravel()
         if ids.size and (ids.min() < 0 or ids.max() >= N):
             raise IndexError("solve id out of range")
-        # ascending and distinct through the mask: 1 ms for 600,000 ids, np.unique 30
+        # ascending and distinct: many of N = 634,000 ids through the mask (4.4 ms for 95% of
+        # them, np.unique 69 to 223), few by sorting them (0.03 ms for 63, the mask's scan 1.3)
         keep = np.zeros(N, np.uint8)
         keep[ids] = 1
-        self.solve_ids = ids = np.flatnonzero(keep)
+        self.solve_ids = ids = np.unique(ids) if ids.size < N // 64 else np.flatnonzero(keep)
         d_keep = _to_dev(keep, torch.uint8, dev)
         sel = L.Select()
         L.check(L.lib().emg_select_init(N, L.ctypes.byref(sel)))
