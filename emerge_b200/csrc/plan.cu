@@ -709,8 +709,8 @@ __global__ void k_chunk_keys(const int32_t *ent_ptr, const Item *items, const do
 }
 
 // Bitonic sort of n2 = 2^m keys. A CTA does every step within a tile of
-// SORT_TILE keys in shared memory: all stages up to the tile (k_sort_tiles), or
-// the steps j < SORT_TILE of stage k (k_sort_tail). The steps between tiles go
+// SORT_TILE keys in shared memory: all stages up to the tile (k_sort_tile<true>), or
+// the steps j < SORT_TILE of stage k (k_sort_tile<false>). The steps between tiles go
 // three to a launch, on the 8 keys a thread exchanges among themselves. 2^14 keys
 // (a port's forcing vector) take 7 launches and 40 us instead of 105 and 176, 2^16
 // and 2^17 30 and 160 us instead of 289 and 510. Tiles of 8,192 keys and 1,024
@@ -953,16 +953,6 @@ int sort_u64(uint64_t *keys, int64_t n2, cudaStream_t s) {
   if (n2 & (n2 - 1)) return fail(EMG_EINVAL, "sort length %lld is not a power of two", (long long)n2);
   if (n2 < 2) return EMG_OK;
   constexpr int smem = SORT_TILE * 8;
-  // the attribute belongs to the current device: set once per device (benign
-  // race: every thread that gets here sets the same value)
-  static bool configured[64] = {false};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
-  if (dev >= 64 || !configured[dev]) {
-    CUDA_TRY(cudaFuncSetAttribute(k_sort_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CUDA_TRY(cudaFuncSetAttribute(k_sort_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    if (dev < 64) configured[dev] = true;
-  }
   const int tiles = grid_for(n2, SORT_TILE);
   k_sort_tile<true><<<tiles, SORT_THREADS, smem, s>>>(keys, n2, 0);
   int rc = launch_check("k_sort_tile");
