@@ -1,7 +1,8 @@
 """Build ``emerge_b200/libemgpu.so`` for sm_100a with nvcc (in-tree).
 
 The element kernel is compiled once per (material kind, precision) from
-``element_inst.cu`` so the six heavy instances build in parallel; everything
+``element_inst.cu``, single and batched launches apart, so the heavy instances
+build in parallel; everything
 is linked into one shared library with a C ABI (``include/emgpu.h``).
 
     python -m emerge_b200.build [--force] [--jobs N]
@@ -38,7 +39,10 @@ def _units():
              ("heat", "heat.cu", ["-fmad=false"])]
     for form in (0, 1, 2):
         for kind in (0, 1, 2):
-            units.append((f"element_{form}_{kind}", "element_inst.cu", [f"-DEMG_FORM={form}", f"-DEMG_KIND={kind}"]))
+            inst = [f"-DEMG_FORM={form}", f"-DEMG_KIND={kind}"]
+            units.append((f"element_{form}_{kind}", "element_inst.cu", inst))
+            units.append((f"element_batch_{form}_{kind}", "element_inst.cu", inst + ["-DEMG_BATCH"]))
+    units.sort(key=lambda u: not u[0].endswith("_2"))  # full tensors take longest: first
     return units
 
 

@@ -45,11 +45,15 @@ enum { FORM_REF64 = 0, FORM_REF32 = 1, FORM_EXACT = 2 };
 // 1.1 KB (diagonal) and 6.9 KB (full). Measured: diagonal at 1,008,000 tets 2,447
 // -> 1,110 us (EXACT 726 -> 660), full at 414,720 1,856 -> 555 (1,276 -> 361).
 // Bound: FP64 latency at eight warps per SM (254 registers).
-// Full tensors go through their symmetric halves first (all there is to a
-// reciprocal material); where a warp has any other, those tets add the
-// antisymmetric halves' part in a second pass (both halves in one pass kept 4.9 KB
-// spilled: 1,607 us).
-enum { KIND_PAIR = 3, KIND_PAIR_FULL = 4, KIND_PAIR_ANTI = 5 };
+// Tets with symmetric tensors (all of a reciprocal material) need only those halves; a
+// warp that has any others goes through these in a pass of their own, with the
+// antisymmetric halves beside the symmetric ones (KIND_PAIR_BOTH). 103,680 tets, none
+// symmetric, packed / block values: FP64 442 / 525 us, exact 270 / 279, against 506 / 485
+// and 336 / 326 for a lane per tet and 895 / 770 and 645 / 479 for a second pass over the
+// whole warp that added the antisymmetric part to the values in memory. Its 14,000
+// instructions do not fit the instruction cache (no-instruction stalls 6.5 of 11.4 cycles
+// per instruction; a symmetric tet's pass 0.6 of 5.6).
+enum { KIND_PAIR = 3, KIND_PAIR_FULL = 4, KIND_PAIR_BOTH = 5 };
 __host__ __device__ constexpr int tensor_kind(int form, int kind) {
   return form == FORM_REF32 || kind == EMG_MAT_ISO ? kind : (kind == EMG_MAT_DIAG ? KIND_PAIR : KIND_PAIR_FULL);
 }
@@ -422,9 +426,31 @@ template <typename R>
 struct Tensors<KIND_PAIR_FULL, R> {
   R G[4][4], H[6][6];
 };
+// G, H of the symmetric halves; the antisymmetric halves' 6 and 15 values above the
+// diagonals lie in shared memory, value i at anti[32 i]: in registers they spilled
+// 4.9 KB beside the moments
+constexpr int ANTI_VALUES = 21;
 template <typename R>
-struct Tensors<KIND_PAIR_ANTI, R> {
+struct Tensors<KIND_PAIR_BOTH, R> {
   R G[4][4], H[6][6];
+  R *anti;
+};
+
+// row-major N x N antisymmetric matrix over its values above the diagonal
+template <int N, typename R>
+struct Anti {
+  const R *v;
+  struct Row {
+    const R *v;
+    int m;
+    __device__ __forceinline__ R operator[](int n) const {
+      if (m == n) return (R)0;
+      const int lo = m < n ? m : n, hi = m < n ? n : m;
+      const R x = v[32 * (lo * (2 * N - 1 - lo) / 2 + hi - lo - 1)];
+      return m < n ? x : -x;
+    }
+  };
+  __device__ __forceinline__ Row operator[](int m) const { return {v, m}; }
 };
 
 __device__ __forceinline__ void cross3(const double a[3], const double b[3], double o[3]) {
@@ -505,7 +531,8 @@ __device__ __forceinline__ void build_cplx(const Geo &Gm, const C64 eps[9], cons
 }
 
 // The lane's part of the forms V b . t a of a 3x3 tensor t (row-major): (e g_m).g_n
-// into G and (u X_P).X_Q into H, of the tensors' symmetric or antisymmetric halves.
+// into G and (u X_P).X_Q into H, of the tensors' symmetric halves and, KIND_PAIR_BOTH,
+// of their antisymmetric ones.
 template <int KIND, typename R>
 __device__ __forceinline__ void build_pair(const Geo &Gm, const double e[9], const double u[9], Tensors<KIND, R> &T) {
   double X[6][3];
@@ -514,38 +541,38 @@ __device__ __forceinline__ void build_pair(const Geo &Gm, const double e[9], con
   for (int p = 0; p < 6; ++p) cross3(Gm.g[pa[p]], Gm.g[pb[p]], X[p]);
   auto form = [&](const double t[9], const double a[3], const double b[3]) {
     double s = 0.0;
-    if constexpr (KIND == KIND_PAIR_ANTI) {  // b . t a = w . (a x b), w = (t21, t02, t10)
-      double c[3];
-      cross3(a, b, c);
-      s = 0.5 * ((t[7] - t[5]) * c[0] + (t[2] - t[6]) * c[1] + (t[3] - t[1]) * c[2]);
-    } else {
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          if (KIND == KIND_PAIR && r != c) continue;
-          const double v = r == c ? t[4 * r] : 0.5 * (t[3 * r + c] + t[3 * c + r]);
-          s += v * (b[r] * a[c]);
-        }
-    }
+      for (int c = 0; c < 3; ++c) {
+        if (KIND == KIND_PAIR && r != c) continue;
+        const double v = r == c ? t[4 * r] : 0.5 * (t[3 * r + c] + t[3 * c + r]);
+        s += v * (b[r] * a[c]);
+      }
     return s * Gm.V;
   };
-  constexpr bool anti = KIND == KIND_PAIR_ANTI;
+  // b . t a = w . (a x b), w = (t21, t02, t10)
+  auto anti = [&](const double t[9], const double a[3], const double b[3]) {
+    double c[3];
+    cross3(a, b, c);
+    return 0.5 * ((t[7] - t[5]) * c[0] + (t[2] - t[6]) * c[1] + (t[3] - t[1]) * c[2]) * Gm.V;
+  };
+  int i = 0;
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
     for (int n = m; n < 4; ++n) {
-      const R v = anti && n == m ? (R)0 : (R)form(e, Gm.g[m], Gm.g[n]);
-      T.G[n][m] = anti ? -v : v;
-      T.G[m][n] = v;
+      T.G[m][n] = T.G[n][m] = (R)form(e, Gm.g[m], Gm.g[n]);
+      if constexpr (KIND == KIND_PAIR_BOTH)
+        if (n > m) T.anti[32 * i++] = (R)anti(e, Gm.g[m], Gm.g[n]);
     }
 #pragma unroll
   for (int p = 0; p < 6; ++p)
 #pragma unroll
     for (int q = p; q < 6; ++q) {
-      const R v = anti && q == p ? (R)0 : (R)form(u, X[p], X[q]);
-      T.H[q][p] = anti ? -v : v;
-      T.H[p][q] = v;
+      T.H[p][q] = T.H[q][p] = (R)form(u, X[p], X[q]);
+      if constexpr (KIND == KIND_PAIR_BOTH)
+        if (q > p) T.anti[32 * i++] = (R)anti(u, X[p], X[q]);
     }
 }
 
@@ -562,7 +589,7 @@ struct EntryT<KIND_PAIR_FULL, R> {
   using T = R;
 };
 template <typename R>
-struct EntryT<KIND_PAIR_ANTI, R> {
+struct EntryT<KIND_PAIR_BOTH, R> {
   using T = R;
 };
 template <typename R>
@@ -581,25 +608,29 @@ __device__ __forceinline__ void scale_sign(CR<double> &x, double s) { x.re *= s,
 template <>
 __device__ __forceinline__ void scale_sign(CR<float> &x, double s) { x.re *= (float)s, x.im *= (float)s; }
 
-// entry (first=f, second=s) of K and M in the canonical frame
-template <int f, int s, int FORM, int KIND, typename R>
-__device__ __forceinline__ void entry(const Tensors<KIND, R> &T, const R *mu, double sig,
-                                      typename EntryT<KIND, R>::T &k, typename EntryT<KIND, R>::T &m) {
-  using E = typename EntryT<KIND, R>::T;
+// entry (first=f, second=s) of K and M in the canonical frame, of the tensors G and H
+template <int f, int s, int FORM, typename E, typename TG, typename TH, typename R>
+__device__ __forceinline__ void contract(const TG &G, const TH &H, const R *mu, double sig, E &k, E &m) {
   E ak{}, am{};
   if constexpr (FORM != FORM_REF64) {
-    emg_tables::Pair<f, s>::stiff(ak, T.H);
-    emg_tables::Pair<f, s>::mass(am, T.G);
+    emg_tables::Pair<f, s>::stiff(ak, H);
+    emg_tables::Pair<f, s>::mass(am, G);
     if (emg_tables::odd(f) != emg_tables::odd(s)) {
       scale_sign(ak, sig);
       scale_sign(am, sig);
     }
   } else {
-    emg_mtables::MPair<f, s>::stiff(ak, T.H, mu);
-    emg_mtables::MPair<f, s>::mass(am, T.G, mu);
+    emg_mtables::MPair<f, s>::stiff(ak, H, mu);
+    emg_mtables::MPair<f, s>::mass(am, G, mu);
   }
   k = ak;
   m = am;
+}
+
+template <int f, int s, int FORM, int KIND, typename R>
+__device__ __forceinline__ void entry(const Tensors<KIND, R> &T, const R *mu, double sig,
+                                      typename EntryT<KIND, R>::T &k, typename EntryT<KIND, R>::T &m) {
+  contract<f, s, FORM>(T.G, T.H, mu, sig, k, m);
 }
 
 // The lane's part of entry (lo, hi). Antisymmetric half: the first function is
@@ -608,7 +639,11 @@ template <int lo, int hi, int FORM, int KIND, typename R>
 __device__ __forceinline__ R pair_value(const Tensors<KIND, R> &T, const R *mu, double sig, uint64_t inv) {
   R k, m;
   entry<lo, hi, FORM, KIND, R>(T, mu, sig, k, m);
-  if (KIND == KIND_PAIR_ANTI && ref_dof(inv, lo) > ref_dof(inv, hi)) return -(k + m);
+  if constexpr (KIND == KIND_PAIR_BOTH && lo != hi) {
+    R ka, ma;
+    contract<lo, hi, FORM>(Anti<4, R>{T.anti}, Anti<6, R>{T.anti + 32 * 6}, mu, sig, ka, ma);
+    return (k + m) + (ref_dof(inv, lo) > ref_dof(inv, hi) ? -(ka + ma) : ka + ma);
+  }
   return k + m;
 }
 
@@ -629,17 +664,6 @@ __device__ __forceinline__ double cfma(double a, double b, double c) { return __
 __device__ __forceinline__ float cfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double cmul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float cmul_rn(float a, float b) { return __fmul_rn(a, b); }
-
-// a staged value into the output: the second pass of a full tensor adds to the first's
-template <int KIND, typename ST>
-__device__ __forceinline__ void put(ST *o, ST v) {
-  if (KIND == KIND_PAIR_ANTI) {
-    const ST was = *o;
-    v.x += was.x;
-    v.y += was.y;
-  }
-  *o = v;
-}
 
 template <int x, int y, int FORM, int KIND, typename R>
 __device__ __forceinline__ void compute_store(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
@@ -674,6 +698,50 @@ __device__ __forceinline__ void compute_store(const Tensors<KIND, R> &T, const R
   row[b] = v;
 }
 
+// A row of KIND_PAIR_BOTH into the stage: entries (x, row_dof<LAYOUT, b>(s)), s < W, at
+// row + s; of the COO block in the reference's order. A group of values is formed before
+// the first is stored, as a store makes the compiler load the antisymmetric halves again.
+template <int FORM>
+__host__ __device__ constexpr int both_group() {
+  return FORM == FORM_REF64 ? 2 : 20;
+}
+
+template <int LAYOUT, int b>
+__host__ __device__ constexpr int row_dof(int s) {
+  return LAYOUT == 0 ? s : (LAYOUT == 1 ? b + s : (s & 1 ? ent_dof2(b + s / 2) : ent_dof1(b + s / 2)));
+}
+
+template <int LAYOUT, int x, int b, int W, int FORM, int s, typename R>
+__device__ __forceinline__ R both_value(const Tensors<KIND_PAIR_BOTH, R> &T, const R *mu, double sig, uint64_t inv) {
+  if constexpr (s < W) {
+    constexpr int y = row_dof<LAYOUT, b>(s);
+    return pair_value<(x < y ? x : y), (x < y ? y : x), FORM, KIND_PAIR_BOTH, R>(T, mu, sig, inv);
+  } else {
+    return (R)0;
+  }
+}
+
+template <int LAYOUT, int x, int b, int W, int FORM, int s0, typename R, int... Ss>
+__device__ __forceinline__ void stage_both_group(const Tensors<KIND_PAIR_BOTH, R> &T, const R *mu, double sig,
+                                                 uint64_t inv, double2 *row, std::integer_sequence<int, Ss...>) {
+  const R v[] = {both_value<LAYOUT, x, b, W, FORM, s0 + Ss, R>(T, mu, sig, inv)...};
+#pragma unroll
+  for (int k = 0; k < both_group<FORM>(); ++k)
+    if (s0 + k < W)
+      reinterpret_cast<R *>(row + (LAYOUT == 0 ? ref_dof(inv, s0 + k) : s0 + k))[threadIdx.x & 1] = v[k];
+}
+
+template <int LAYOUT, int x, int b, int W, int FORM, typename R, int... Gs>
+__device__ __forceinline__ void stage_both_row(const Tensors<KIND_PAIR_BOTH, R> &T, const R *mu, double sig,
+                                               uint64_t inv, double2 *row, std::integer_sequence<int, Gs...>) {
+  (stage_both_group<LAYOUT, x, b, W, FORM, both_group<FORM>() * Gs, R>(
+       T, mu, sig, inv, row, std::make_integer_sequence<int, both_group<FORM>()>{}),
+   ...);
+}
+
+template <int W, int FORM>
+using both_groups = std::make_integer_sequence<int, (W + both_group<FORM>() - 1) / both_group<FORM>()>;
+
 template <int x, int FORM, int KIND, typename R, int... Ys>
 __device__ __forceinline__ void compute_row(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
                                             const CR<R> &cM, uint64_t inv, int rx, typename StoreT<R>::T *row,
@@ -688,9 +756,13 @@ __device__ __forceinline__ void do_row(const Tensors<KIND, R> &T, const R *mu, d
   constexpr int LPT = lanes_per_tet(KIND);
   const int lane = threadIdx.x & 31;
   const int rx = ref_dof(inv, X);
-  if (active)
-    compute_row<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, rx, stage + lane / LPT * 21,
-                                  std::make_integer_sequence<int, 20>{});
+  if (active) {
+    if constexpr (KIND == KIND_PAIR_BOTH)
+      stage_both_row<0, X, 0, 20, FORM, R>(T, mu, sig, inv, stage + lane / LPT * 21, both_groups<20, FORM>{});
+    else
+      compute_row<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, rx, stage + lane / LPT * 21,
+                                    std::make_integer_sequence<int, 20>{});
+  }
   __syncwarp();
   // cooperative, coalesced write of the warp's rows (one of 20 contiguous values per tet)
 #pragma unroll 1
@@ -700,7 +772,7 @@ __device__ __forceinline__ void do_row(const Tensors<KIND, R> &T, const R *mu, d
     int ia_r = __shfl_sync(0xffffffffu, ia, r * LPT);
     int a_r = __shfl_sync(0xffffffffu, rx, r * LPT);
     bool act_r = __shfl_sync(0xffffffffu, (int)active, r * LPT);
-    if (act_r) put<KIND>(out + (int64_t)ia_r * 400 + a_r * 20 + c, stage[r * 21 + c]);
+    if (act_r) out[(int64_t)ia_r * 400 + a_r * 20 + c] = stage[r * 21 + c];
   }
   __syncwarp();
 }
@@ -768,9 +840,13 @@ __device__ __forceinline__ void do_row_packed(const Tensors<KIND, R> &T, const R
                                               typename StoreT<R>::T *stage, typename StoreT<R>::T *out) {
   constexpr int W = 20 - X, LPT = lanes_per_tet(KIND);
   const int lane = threadIdx.x & 31;
-  if (active)
-    compute_row_packed<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane / LPT * (W | 1),
-                                         std::make_integer_sequence<int, W>{});
+  if (active) {
+    if constexpr (KIND == KIND_PAIR_BOTH)
+      stage_both_row<1, X, X, W, FORM, R>(T, mu, sig, inv, stage + lane / LPT * (W | 1), both_groups<W, FORM>{});
+    else
+      compute_row_packed<X, FORM, KIND, R>(T, mu, sig, cK, cM, inv, stage + lane / LPT * (W | 1),
+                                           std::make_integer_sequence<int, W>{});
+  }
   // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
   const unsigned act = __ballot_sync(0xffffffffu, active);
   const int64_t ia_w = (int64_t)ia - lane / LPT;
@@ -778,7 +854,7 @@ __device__ __forceinline__ void do_row_packed(const Tensors<KIND, R> &T, const R
 #pragma unroll 2
   for (int e = lane; e < 32 / LPT * W; e += 32) {
     const int r = e / W, c = e - r * W;
-    if ((act >> (r * LPT)) & 1u) put<KIND>(out + (ia_w + r) * 210 + packed_index(X, X) + c, stage[r * (W | 1) + c]);
+    if ((act >> (r * LPT)) & 1u) out[(ia_w + r) * 210 + packed_index(X, X) + c] = stage[r * (W | 1) + c];
   }
   __syncwarp();
 }
@@ -892,6 +968,44 @@ __device__ __forceinline__ void stage_block_row(const Tensors<KIND, R> &T, const
    ...);
 }
 
+// HALF 0, 1: the first, the second DoF's entries of block row I (KIND_PAIR_BOTH); 2: both
+template <int FORM, int KIND, typename R, int I, int HALF>
+__device__ __forceinline__ void store_pair_row(const Tensors<KIND, R> &T, const R *mu, double sig, uint64_t inv,
+                                               bool active, int ia, bool wide, double2 *stage, double2 *out) {
+  // V values at a time
+  constexpr int W = (HALF == 2 ? 4 : 2) * (10 - I), LPT = lanes_per_tet(KIND), V = KIND == KIND_PAIR ? 2 : 1;
+  constexpr int ROUNDS = W / LPT / V;
+  static_assert(W % (LPT * V) == 0, "whole rounds of the warp");
+  const int lane = threadIdx.x & 31;
+  if (active) {
+    if constexpr (HALF == 2)
+      stage_block_row<I, FORM, KIND, R>(T, mu, sig, inv, stage + lane / LPT * (W | 1),
+                                        std::make_integer_sequence<int, 10 - I>{});
+    else
+      stage_both_row<2, HALF ? ent_dof2(I) : ent_dof1(I), I, W, FORM, R>(T, mu, sig, inv, stage + lane / LPT * (W | 1),
+                                                                         both_groups<W, FORM>{});
+  }
+  // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
+  const unsigned act = __ballot_sync(0xffffffffu, active);
+  const int64_t ia_w = (int64_t)ia - lane / LPT;
+  __syncwarp();
+#pragma unroll 2
+  for (int it = 0; it < ROUNDS; ++it) {
+    const int e = it * 32 + lane;
+    const int r = e / (W / V), c = V * (e - r * (W / V));
+    if ((act >> (r * LPT)) & 1u) {
+      const int at = HALF == 2 ? c : 2 * HALF + 4 * (c / 2) + (c & 1);
+      double2 *o = out + (ia_w + r) * kBlockValues + 4 * block_index(I, I) + at;
+      const double2 *v = stage + r * (W | 1) + c;
+      if constexpr (V == 2)
+        store_half(o, v[0], v[1], wide);
+      else
+        *o = v[0];
+    }
+  }
+  __syncwarp();
+}
+
 template <int FORM, int KIND, typename R, int I>
 __device__ __forceinline__ void do_row_block(const Tensors<KIND, R> &T, const R *mu, double sig, const CR<R> &cK,
                                              const CR<R> &cM, uint64_t inv, bool active, int ia, bool wide,
@@ -901,32 +1015,11 @@ __device__ __forceinline__ void do_row_block(const Tensors<KIND, R> &T, const R 
       BlockRow<FORM, KIND, R>{T, mu, sig, cK, cM, inv, wide}.template store<I>(
           out + (int64_t)ia * kBlockValues + 4 * block_index(I, I), std::make_integer_sequence<int, 10 - I>{});
     __syncwarp();  // the compiler would otherwise form products of later rows ahead, and spill them
+  } else if constexpr (KIND == KIND_PAIR_BOTH) {
+    store_pair_row<FORM, KIND, R, I, 0>(T, mu, sig, inv, active, ia, wide, stage, out);
+    store_pair_row<FORM, KIND, R, I, 1>(T, mu, sig, inv, active, ia, wide, stage, out);
   } else {
-    // V values at a time
-    constexpr int W = 4 * (10 - I), LPT = lanes_per_tet(KIND), V = KIND == KIND_PAIR ? 2 : 1, ROUNDS = W / LPT / V;
-    static_assert(W % (LPT * V) == 0, "whole rounds of the warp");
-    const int lane = threadIdx.x & 31;
-    if (active)
-      stage_block_row<I, FORM, KIND, R>(T, mu, sig, inv, stage + lane / LPT * (W | 1),
-                                        std::make_integer_sequence<int, 10 - I>{});
-    // the warp's tets are consecutive assembled indices: the r-th one's is ia - lane / LPT + r
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    const int64_t ia_w = (int64_t)ia - lane / LPT;
-    __syncwarp();
-#pragma unroll 2
-    for (int it = 0; it < ROUNDS; ++it) {
-      const int e = it * 32 + lane;
-      const int r = e / (W / V), c = V * (e - r * (W / V));
-      if ((act >> (r * LPT)) & 1u) {
-        double2 *o = out + (ia_w + r) * kBlockValues + 4 * block_index(I, I) + c;
-        const double2 *v = stage + r * (W | 1) + c;
-        if constexpr (V == 2)
-          store_half(o, v[0], v[1], wide);
-        else
-          put<KIND>(o, v[0]);
-      }
-    }
-    __syncwarp();
+    store_pair_row<FORM, KIND, R, I, 2>(T, mu, sig, inv, active, ia, wide, stage, out);
   }
 }
 
@@ -945,7 +1038,16 @@ __device__ __forceinline__ void all_rows_block(const Tensors<KIND, R> &T, const 
 // of one value position fall in distinct shared-memory bank groups
 template <int LAYOUT, int TK>
 __host__ __device__ constexpr int stage_values() {
-  return LAYOUT != 2 ? 21 : (TK >= KIND_PAIR ? 41 : 0);
+  return LAYOUT != 2 ? 21 : (TK == KIND_PAIR_BOTH ? 21 : (TK >= KIND_PAIR ? 41 : 0));
+}
+
+// shared memory of a warp: its tets' staged rows; for full tensors in pairs at least the
+// rows and the antisymmetric halves of KIND_PAIR_BOTH (which stages half block rows)
+template <int LAYOUT, int TK, typename ST>
+__host__ __device__ constexpr size_t stage_bytes() {
+  const size_t rows = (size_t)32 / lanes_per_tet(TK) * stage_values<LAYOUT, TK>() * sizeof(ST);
+  const size_t both = (size_t)16 * stage_values<LAYOUT, KIND_PAIR_BOTH>() * sizeof(ST) + 32 * ANTI_VALUES * sizeof(double);
+  return TK == KIND_PAIR_FULL && both > rows ? both : rows;
 }
 
 // LAYOUT 0: the reference's COO block [ia][a][b] (400 values, each entry
@@ -955,18 +1057,18 @@ __host__ __device__ constexpr int stage_values() {
 // LAYOUT 2: the entity-pair blocks [ia][220] (the assembly path)
 // One CTA's tets (elem_tets_per_cta), from assembled index ia0 of the job a on
 // (every thread of the CTA calls it with the same ia0).
-// TK: the tensors' form. Returns whether any tet of the warp needs the
-// antisymmetric pass.
+// TK: the tensors' form; mine: whether this lane's tet takes part.
 template <int FORM, int KIND, int LAYOUT, int TK>
-__device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, unsigned rows, unsigned char *stage_raw) {
+__device__ __forceinline__ void element_pass(const ElemArgs &a, int64_t ia0, bool mine, unsigned rows,
+                                             unsigned char *stage_raw) {
   using R = typename FormReal<FORM>::T;
   using ST = typename StoreT<R>::T;
   constexpr int LPT = lanes_per_tet(TK);
-  constexpr int STAGE = stage_values<LAYOUT, TK>();
-  ST *stage = reinterpret_cast<ST *>(stage_raw) + (threadIdx.x >> 5) * (32 / LPT * STAGE);
+  unsigned char *const shared = stage_raw + (threadIdx.x >> 5) * stage_bytes<LAYOUT, tensor_kind(FORM, KIND), ST>();
+  ST *stage = reinterpret_cast<ST *>(shared);
   ST *out = reinterpret_cast<ST *>(a.out);
   const int64_t ia64 = ia0 + threadIdx.x / LPT;
-  bool active = ia64 < a.nA;
+  bool active = mine && ia64 < a.nA;
   const int ia = (int)ia64;
   Geo G;
   Tensors<TK, R> T;
@@ -978,7 +1080,8 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
   CR<R> cK{0, 0}, cM{0, 0};
   double sig = 1.0;
   uint64_t inv = 0;
-  bool asym = false;
+  if constexpr (TK == KIND_PAIR_BOTH)
+    T.anti = reinterpret_cast<R *>(shared + 32 / LPT * stage_values<LAYOUT, TK>() * sizeof(ST)) + (threadIdx.x & 31);
   if (active) {
     int64_t it = a.tetids ? (int64_t)a.tetids[ia] : ia64;
     int64_t v[4];
@@ -1033,14 +1136,6 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
             }
           matinv3(mu3, minv);
           if constexpr (LPT == 2) {
-            auto symmetric = [](const C64 t[9]) {
-              return t[1].re == t[3].re && t[1].im == t[3].im && t[2].re == t[6].re && t[2].im == t[6].im &&
-                     t[5].re == t[7].re && t[5].im == t[7].im;
-            };
-            asym = KIND == EMG_MAT_FULL && !(symmetric(eps) && symmetric(mu3));
-            // a reciprocal tet keeps the first pass's values whatever its neighbours are:
-            // the inverse of its mu may be symmetric only up to rounding
-            if (TK == KIND_PAIR_ANTI) active = asym;
             double e[9], u[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
@@ -1071,16 +1166,40 @@ __device__ __forceinline__ bool element_pass(const ElemArgs &a, int64_t ia0, uns
     all_rows_packed<FORM, TK, R>(T, mu, sig, cK, cM, inv, active, ia, stage, out,
                                    std::make_integer_sequence<int, 20>{});
   }
-  return TK == KIND_PAIR_FULL && __any_sync(0xffffffffu, asym);
 }
 
-// rows: bit i set to write block row i (block layout; the others write all rows)
+// Whether a tensor of the lane's tet is not symmetric; the even lane of a pair looks at
+// its eps, the odd one at its mu.
+__device__ __forceinline__ bool not_reciprocal(const ElemArgs &a, int64_t ia) {
+  bool other = false;
+  const double2 *t = static_cast<const double2 *>((threadIdx.x & 1) ? a.ur : a.er);
+  const int64_t it = ia < a.nA ? (a.tetids ? (int64_t)a.tetids[ia] : ia) : -1;
+  if (t && it >= 0 && it < a.nT) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int rc[3] = {1, 2, 5}, cr[3] = {3, 6, 7};
+      const double2 x = __ldg(t + rc[i] * a.nT + it), y = __ldg(t + cr[i] * a.nT + it);
+      other = other || x.x != y.x || x.y != y.y;
+    }
+  }
+  return __shfl_xor_sync(0xffffffffu, (int)other, 1) || other;
+}
+
+// rows: bit i set to write block row i (block layout; the others write all rows).
+// Full tensors in pairs: a tet's pass depends on its own tensors alone, so its values
+// are the same whatever its neighbours are.
 template <int FORM, int KIND, int LAYOUT>
 __device__ __forceinline__ void element_cta(const ElemArgs &a, int64_t ia0, unsigned rows, unsigned char *stage_raw) {
   constexpr int TK = tensor_kind(FORM, KIND);
-  const bool asym = element_pass<FORM, KIND, LAYOUT, TK>(a, ia0, rows, stage_raw);
-  if constexpr (TK == KIND_PAIR_FULL)
-    if (asym) element_pass<FORM, KIND, LAYOUT, KIND_PAIR_ANTI>(a, ia0, rows, stage_raw);
+  if constexpr (TK == KIND_PAIR_FULL) {
+    const int64_t ia = ia0 + threadIdx.x / 2;
+    const bool other = not_reciprocal(a, ia);
+    if (__any_sync(0xffffffffu, !other && ia < a.nA))
+      element_pass<FORM, KIND, LAYOUT, TK>(a, ia0, !other, rows, stage_raw);
+    if (__any_sync(0xffffffffu, other)) element_pass<FORM, KIND, LAYOUT, KIND_PAIR_BOTH>(a, ia0, other, rows, stage_raw);
+  } else {
+    element_pass<FORM, KIND, LAYOUT, TK>(a, ia0, true, rows, stage_raw);
+  }
 }
 
 // A mesh that leaves SMs idle: its tets are gone through by several CTAs,
@@ -1145,8 +1264,7 @@ __global__ void __launch_bounds__(ELEM_THREADS, elem_min_blocks<FORM, KIND>())
 template <int FORM, int KIND, int LAYOUT>
 int launch_element_t(const ElemArgs &a, cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
-  constexpr size_t smem =
-      (size_t)elem_tets<FORM, KIND>() * stage_values<LAYOUT, tensor_kind(FORM, KIND)>() * sizeof(ST);
+  constexpr size_t smem = ELEM_THREADS / 32 * stage_bytes<LAYOUT, tensor_kind(FORM, KIND), ST>();
   static_assert(elem_tets<FORM, KIND>() == elem_tets_per_cta(FORM, KIND), "the host's table of CTAs");
   // the attribute belongs to the current device: set once per device (benign
   // race: every thread that gets here sets the same value)
@@ -1173,8 +1291,7 @@ template <int FORM, int KIND, int LAYOUT>
 int launch_element_batch_t(const ElemArgs *d_jobs, const int64_t *d_cta_start, int n_jobs, int64_t total_ctas,
                            cudaStream_t s) {
   using ST = typename StoreT<typename FormReal<FORM>::T>::T;
-  constexpr size_t smem =  // element_cta's stage
-      (size_t)elem_tets<FORM, KIND>() * stage_values<LAYOUT, tensor_kind(FORM, KIND)>() * sizeof(ST);
+  constexpr size_t smem = ELEM_THREADS / 32 * stage_bytes<LAYOUT, tensor_kind(FORM, KIND), ST>();
   static bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
