@@ -1223,7 +1223,7 @@ __device__ __forceinline__ unsigned part_rows(int part, int n_parts) {
 
 // CTAs per SM the compiler must fit. The isotropic FP64 forms at their natural
 // 232-255 registers (two CTAs) beat every cap (three CTAs, 2.01M tets: 1.84 ->
-// 3.68 ms, 1.9 KB of spills); the mixed form takes 90-254 (five CTAs per SM for the
+// 3.68 ms, 1.9 KB of spills); the mixed form takes 88-254 (five CTAs per SM for the
 // isotropic instance; held to six or seven, 1.008M tets: 362 -> 375 / 385 us).
 template <int FORM, int KIND>
 constexpr int elem_min_blocks() {
