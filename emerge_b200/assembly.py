@@ -66,14 +66,16 @@ def _empty(numel: int, dtype: torch.dtype, dev: torch.device, alloc=None) -> tor
 _TURN_ON_DEVICE = 65536
 
 
-def _to_dev(a: np.ndarray, dtype: torch.dtype, dev: torch.device, alloc=None) -> torch.Tensor:
+def _to_dev(a: np.ndarray, dtype: torch.dtype, dev: torch.device, alloc=None, wait: bool = True) -> torch.Tensor:
+    """The array on the device. It may be read on any stream once this returns;
+    without ``wait`` only on the current one (or after it)."""
     if alloc is None:
         if (isinstance(a, np.ndarray) and a.ndim == 2 and a.flags.f_contiguous and not a.flags.c_contiguous
                 and a.flags.writeable and a.size >= _TURN_ON_DEVICE):
-            # laid out the other way round: uploaded as it is and turned over there;
-            # done before this returns, as a plain upload is, whatever stream reads it next
+            # laid out the other way round: uploaded as it is and turned over there
             t = torch.from_numpy(a.T).to(device=dev, dtype=dtype, non_blocking=False).T.contiguous()
-            torch.cuda.current_stream(dev).synchronize()
+            if wait:
+                torch.cuda.current_stream(dev).synchronize()
             return t
         return torch.from_numpy(np.ascontiguousarray(a)).to(device=dev, dtype=dtype, non_blocking=False)
     h = np.ascontiguousarray(a, dtype=_NP[dtype])
