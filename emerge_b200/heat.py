@@ -16,6 +16,8 @@ COO -> CSC one (``GpuCOOMapping``), also usable for any other slot list.
 """
 from __future__ import annotations
 
+import copy
+
 import numpy as np
 import torch
 from scipy.sparse import csc_matrix
@@ -35,6 +37,18 @@ class Legrange2:
         self.n_field = int(mesh.n_nodes + mesh.n_edges)
         self.tet_to_field = np.concatenate([np.asarray(mesh.tets), np.asarray(mesh.tet_to_edge) + mesh.n_nodes]
                                            ).astype(np.int64)
+
+
+def _outside(a: np.ndarray, n: int) -> bool:
+    """Whether any of the indices lies outside [0, n). The usual types through torch,
+    which looks at them once and on all host threads (1.4M int64: 0.2 ms, numpy 0.9)."""
+    if not a.size:
+        return False
+    if a.dtype in (np.dtype(np.int32), np.dtype(np.int64)):
+        lo, hi = torch.aminmax(torch.from_numpy(np.ascontiguousarray(a)))
+    else:
+        lo, hi = a.min(), a.max()
+    return bool(lo < 0) or bool(hi >= n)
 
 
 class CooValues:
@@ -170,7 +184,7 @@ class GpuCOOMapping:
         dev = _device(device)
         t2f = np.asarray(tet_to_field)
         D, nT = t2f.shape
-        if t2f.size and (t2f.min() < 0 or t2f.max() >= N):
+        if _outside(t2f, N):
             raise IndexError("tet_to_field entry outside [0, N)")
         dofs = _to_dev(t2f, torch.int32, dev).t().contiguous()  # a tet's DoFs side by side
         lib = L.lib()
@@ -234,16 +248,26 @@ class GpuCOOMapping:
         return csc_matrix((vals, self.indices, self.indptr), shape=(self.N, self.N))
 
 
-def _bits(a: np.ndarray) -> torch.Tensor:
-    """A host array's values bit for bit, as a torch tensor (its copies and
-    comparisons use all host threads)."""
-    b = np.ascontiguousarray(a).reshape(-1)
-    return torch.from_numpy(b.view(np.int64 if b.nbytes % 8 == 0 else np.uint8))
+class _HostCopy:
+    """An array's values as they were, to tell whether it still holds them (bit
+    by bit; torch's copies and comparisons use all host threads)."""
+
+    def __init__(self, a: np.ndarray):
+        self.dtype, self.shape, self.bits = a.dtype, a.shape, self._bits(a).clone()
+
+    @staticmethod
+    def _bits(a: np.ndarray) -> torch.Tensor:
+        b = np.ascontiguousarray(a).reshape(-1)
+        return torch.from_numpy(b.view(np.int64 if b.nbytes % 8 == 0 else np.uint8))
+
+    def same(self, a: np.ndarray) -> bool:
+        return a.dtype == self.dtype and a.shape == self.shape and torch.equal(self._bits(a), self.bits)
 
 
-class _HeatTopology:
-    """Tets and the COO mapping of one field, kept on the device with host
-    copies of the arrays that they were made from."""
+class _HeatMesh:
+    """Nodes, tets and the COO mapping of one field, kept on the device for its
+    stiffness and mass calls with host copies of the arrays that they were made
+    from."""
 
     def __init__(self, field, tets: np.ndarray, t2f: np.ndarray, n_nodes: int, device):
         if t2f.ndim != 2 or t2f.shape[0] != 10:
@@ -251,11 +275,11 @@ class _HeatTopology:
         self.n_tets = int(tets.shape[1])
         if t2f.shape[1] != self.n_tets:
             raise ValueError("tet_to_field and mesh.tets differ in tet count")
-        if tets.size and (tets.min() < 0 or tets.max() >= n_nodes):  # before narrowing to int32
+        if _outside(tets, n_nodes):  # before narrowing to int32
             raise IndexError("tet node index outside [0, n_nodes)")
-        self.field = field
+        self.field, self.n_nodes = field, n_nodes
         self.sizes = (n_nodes, int(field.n_field), device)
-        self.made_from = [(a.dtype, a.shape, _bits(a).clone()) for a in (tets, t2f)]
+        self.made_from = (_HostCopy(tets), _HostCopy(t2f))
         self.tets = _to_dev(tets, torch.int32, device)
         self.cmap = GpuCOOMapping.from_tet_to_field(t2f, int(field.n_field), device)
 
@@ -263,26 +287,21 @@ class _HeatTopology:
         """Whether it was made of this field as the field's arrays are now. They
         are compared value by value: a partitioned field may be renumbered in
         place, and an array's id is given to the next one once it is gone."""
-        if self.field is not field or self.sizes != (n_nodes, int(field.n_field), device):
-            return False
-        return all(a.dtype == dtype and a.shape == shape and torch.equal(_bits(a), bits)
-                   for a, (dtype, shape, bits) in zip((tets, t2f), self.made_from))
+        return (self.field is field and self.sizes == (n_nodes, int(field.n_field), device)
+                and self.made_from[0].same(tets) and self.made_from[1].same(t2f))
+
+    def at(self, nodes: np.ndarray) -> "_HeatMesh":
+        """The same topology with the coordinates as they are now."""
+        h = copy.copy(self)
+        if "nodes" not in vars(h) or not h.nodes_from.same(nodes):
+            h.nodes_from, h.nodes = _HostCopy(nodes), _to_dev(nodes, torch.float64, h.sizes[2])
+        return h
 
 
-class _HeatMesh:
-    """Nodes, tets and the COO mapping for one call."""
-
-    def __init__(self, topology: _HeatTopology, nodes: torch.Tensor, n_nodes: int):
-        self.n_nodes, self.n_tets, self.nodes = n_nodes, topology.n_tets, nodes
-        self.tets, self.cmap = topology.tets, topology.cmap
-
-
-_KEPT: _HeatTopology | None = None
+_KEPT: _HeatMesh | None = None
 
 
 def _heat_mesh(field, device) -> _HeatMesh:
-    """The coordinates are uploaded on every call; tets and mapping are kept for
-    the stiffness and mass calls of a field."""
     global _KEPT
     dev, m = _device(device), field.mesh
     if dev.index is None:
@@ -291,8 +310,9 @@ def _heat_mesh(field, device) -> _HeatMesh:
     kept = _KEPT
     if kept is None or not kept.fits(field, tets, t2f, n_nodes, dev):
         kept = _KEPT = None  # one field resident at a time
-        kept = _KEPT = _HeatTopology(field, tets, t2f, n_nodes, dev)
-    return _HeatMesh(kept, _to_dev(np.asarray(m.nodes, dtype=np.float64), torch.float64, dev), n_nodes)
+        kept = _HeatMesh(field, tets, t2f, n_nodes, dev)
+    kept = _KEPT = kept.at(np.asarray(m.nodes, dtype=np.float64))
+    return kept
 
 
 def _element(field, coef: np.ndarray, kind: int, precision: str, device) -> tuple[CooValues, GpuCOOMapping]:
