@@ -60,7 +60,8 @@ class FieldOnDevice:
         """The solution x at points f8[3, n] inside tets tet_of (int, -1 =
         outside -> NaN): complex128 [3, n] on the device."""
         xd = self._x(x)
-        pts = _to_dev(np.asarray(points, dtype=np.float64), torch.float64, self.device, wait=False)  # read on this stream
+        # read on this stream: not waited for
+        pts = _to_dev(np.asarray(points, dtype=np.float64), torch.float64, self.device, wait=False)
         tt = _to_dev(np.asarray(tet_of, dtype=np.int64), torch.int32, self.device)
         n = int(pts.shape[1])
         out = torch.empty((3, n), dtype=torch.complex128, device=self.device)
